@@ -1,8 +1,9 @@
 """Build the CUDA library (libcubature_b200.so) in-tree for sm_100a.
 
-Compiles old-gpuintegration_b200/csrc/capi.cu and one instantiation unit per
-dimension (capi_dim.cu with -DCUB_DIM=N) in parallel with nvcc, then links a
-shared library next to the Python package.  Objects are rebuilt only when a
+Compiles old-gpuintegration_b200/csrc/capi.cu and the instantiation units of
+capi_dim.cu (one per dimension and integrand family, -DCUB_DIM=N
+-DCUB_FAMILY=F, and a dispatch unit per dimension) in parallel with nvcc, then
+links a shared library next to the Python package.  Objects are rebuilt only when a
 source or header is newer.
 
     python old-gpuintegration_b200/build.py [--jobs J] [--verbose]
@@ -24,11 +25,15 @@ INCLUDE = ROOT / "include"
 OBJ = PKG / "_build"
 LIB = PKG / "cubature" / "libcubature_b200.so"
 DIMS = range(2, 9)
+FAMILIES = ["Gaussian", "Oscillatory", "CornerPeak", "ProductPeak", "Continuous",
+            "Discontinuous", "CosSum"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + [
     "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
     "--expt-relaxed-constexpr", f"-I{INCLUDE}", f"-I{CSRC}",
+    # by itself nvcc compresses only the larger units' device code
+    "-Xfatbin", "-compress-all",
 ]
 
 
@@ -44,22 +49,28 @@ def _deps() -> list[Path]:
                   list(INCLUDE.rglob("*.cuh")) + list(CSRC.glob("*.h")))
 
 
+# headers that one source alone includes
+ONLY = {"mlp.cuh": "mlp.cu", "umma.cuh": "mlp.cu"}
+
+
 def _stale(obj: Path, src: Path, deps: list[Path]) -> bool:
     if not obj.exists():
         return True
     t = obj.stat().st_mtime
-    return any(p.stat().st_mtime > t for p in [src, *deps])
+    return any(p.stat().st_mtime > t for p in [src, *deps] if ONLY.get(p.name, src.name) == src.name)
 
 
 def units() -> list[tuple[Path, Path, list[str]]]:
-    out = [(CSRC / "capi.cu", OBJ / "capi.o", []),
-           (CSRC / "noalloc.cu", OBJ / "noalloc.o", []),
-           (CSRC / "peak.cu", OBJ / "peak.o", []),
-           (CSRC / "capi_tables.cu", OBJ / "capi_tables.o", []),
-           (CSRC / "graph.cu", OBJ / "graph.o", []),
+    # the slowest first, so that the last jobs of a parallel build are short
+    out = [(CSRC / "capi_tables.cu", OBJ / "capi_tables.o", []),
            (CSRC / "mlp.cu", OBJ / "mlp.o", [])]
-    for n in DIMS:
+    for n in sorted(DIMS, reverse=True):
         out.append((CSRC / "capi_dim.cu", OBJ / f"capi_dim{n}.o", [f"-DCUB_DIM={n}"]))
+        for f in FAMILIES:
+            out.append((CSRC / "capi_dim.cu", OBJ / f"capi_dim{n}_{f}.o",
+                        [f"-DCUB_DIM={n}", f"-DCUB_FAMILY={f}"]))
+    for name in ("capi", "noalloc", "peak", "graph"):
+        out.append((CSRC / f"{name}.cu", OBJ / f"{name}.o", []))
     return out
 
 
