@@ -142,6 +142,7 @@ class Workspace {
     avg = err = nullptr;
     axis = active = chunk_excl = nullptr;
     part = nullptr;
+    tile = nullptr;
     chunk_cnt = int_cnt = nullptr;
     axis_alt = excl_alt = chunk_int = nullptr;
     avg_alt = err_alt = nullptr;
@@ -183,6 +184,7 @@ class Workspace {
   int* active = nullptr;
   ChunkPartial* part = nullptr;
   int* chunk_excl = nullptr;
+  TileSum* tile = nullptr;
   unsigned* chunk_cnt = nullptr;
   // second parity of the persistent kernel's lazy split
   int* axis_alt = nullptr;
@@ -288,6 +290,7 @@ class Workspace {
     if (!alloc(&avg, sizeof(double) * ncap) || !alloc(&err, sizeof(double) * ncap) ||
         !alloc(&axis, sizeof(int) * ncap) || !alloc(&active, sizeof(int) * ncap) ||
         !alloc(&part, sizeof(ChunkPartial) * nchunk) || !alloc(&chunk_excl, sizeof(int) * nchunk) ||
+        !alloc(&tile, sizeof(TileSum) * (nchunk / kTileChunks + 1)) ||
         !alloc(&chunk_cnt, sizeof(unsigned) * nchunk) || !alloc(&axis_alt, sizeof(int) * ncap) ||
         !alloc(&excl_alt, sizeof(int) * nchunk) || !alloc(&cmask, sizeof(unsigned) * 2 * nchunk) ||
         !alloc(&chunk_int, sizeof(int) * nchunk) || !alloc(&avg_alt, sizeof(double) * ncap) ||
@@ -312,6 +315,7 @@ class Workspace {
     } else {
       ncap = std::max<long long>(slots, left_cap_ * 2);
     }
+    ncap = (ncap + 31) & ~31ll;  // children are stored as 16-byte pairs
     double *nlo = nullptr, *nlen = nullptr;
     int* nrid = nullptr;
     LeftoverResult* nres = nullptr;
@@ -372,6 +376,7 @@ class Workspace {
     free_buf(active);
     free_buf(part);
     free_buf(chunk_excl);
+    free_buf(tile);
     free_buf(chunk_cnt);
     free_buf(axis_alt);
     free_buf(excl_alt);
@@ -431,6 +436,7 @@ class Workspace {
     if (bytes <= slab_bytes_ && heap_ints <= heap_ints_) return true;
     free_buf(slab);
     free_buf(heap);
+    slab_bytes_ = heap_ints_ = 0;
     if (!alloc(&slab, bytes) || !alloc(&heap, sizeof(int) * heap_ints)) return false;
     slab_bytes_ = bytes;
     heap_ints_ = heap_ints;
@@ -708,10 +714,24 @@ inline int grid_divisions(int ndim) { return ndim > 10 ? 1 : (ndim >= 5 ? 2 : 4)
 template <int N, int K, class Src>
 inline void launch_eval(const Src& src, const RuleTables& T, const EngineArgs& a, int sms,
                         cudaStream_t s) {
+  constexpr int kThreads = kEvalThreads<K, detail::SourceFn<Src>>;
   const long long threads = (long long)a.n * K;
-  long long blocks = (threads + 255) / 256;
+  long long blocks = (threads + kThreads - 1) / kThreads;
   blocks = std::max<long long>(1, std::min<long long>(blocks, (long long)sms * 32));
-  k_eval<N, K, Src><<<(unsigned)blocks, 256, 0, s>>>(src, T, a);
+  k_eval<N, K, Src><<<(unsigned)blocks, kThreads, 0, s>>>(src, T, a);
+}
+
+// List lengths from which the multi-launch rule kernel takes one lane and 8
+// lanes per region (below: 32).  Point by point, one lane needs a list that
+// fills the chip (512 regions an SM); a factored integrand (kFactored) costs
+// a tenth of that per region, and one lane is always the faster.
+struct EvalLanes {
+  int k1_min, k8_min;
+};
+template <class Src>
+inline EvalLanes eval_lanes(int sms) {
+  if (detail::kFactored<detail::SourceFn<Src>>) return {0, 0};
+  return {sms * 512, sms * 64};
 }
 
 namespace detail {
@@ -826,6 +846,7 @@ inline void bind_lists(const Workspace& ws, EngineArgs& a, int cur, long long n)
   a.active = ws.active;
   a.part = ws.part;
   a.chunk_excl = ws.chunk_excl;
+  a.tile = ws.tile;
   a.chunk_cnt = ws.chunk_cnt;
   a.int_cnt = ws.int_cnt;
   a.nlo = ws.lo[cur ^ 1];
@@ -844,6 +865,7 @@ inline PersistArgs persist_args(const Workspace& ws, const EngineArgs& a, const 
                                 const double* d_box) {
   PersistArgs p;
   p.base = a;
+  p.base.tile = nullptr;  // its lists are short
   const long long nchunk = ws.cap() / 32 + 1;
   for (int b = 0; b < 2; ++b) {
     p.lo[b] = ws.lo[b];
@@ -932,8 +954,8 @@ inline void persistent_control(Workspace& ws, const IterState& hs, int cur) {
 namespace detail {
 
 // The device-driven loop of dimension N and integrand source Src, built on
-// first use: WHILE { bind; SWITCH { rule with 1 | 8 | 32 lanes per region };
-// partials; decide; scan; split; advance; test }.  Grids are the largest
+// first use: WHILE { bind; SWITCH { rule with 1 lane per region | 8 lanes,
+// partials | 32 lanes, partials }; tiles; decide; scan; split; advance; test }.  Grids are the largest
 // the host-driven loop uses for the lane count or step (the kernels stride
 // over the list).  Null when a graph with conditional nodes cannot be built
 // here; the host then drives the iterations.
@@ -981,8 +1003,10 @@ Workspace::LoopEntry* loop_graph(Workspace& ws, int sms) {
   const RuleTables T = make_rule9_tables(N);
   void* a_eval[] = {(void*)&lac, (void*)&T};
   void* a_test[] = {(void*)&lac, (void*)&again};
-  cudaGraphNode_t n_bind = nullptr, n_sw = nullptr, n_part = nullptr, n_dec = nullptr,
-                  n_scan = nullptr, n_split = nullptr, n_adv = nullptr, n_test = nullptr, n_ev;
+  cudaGraphNode_t n_bind = nullptr, n_sw = nullptr, n_tile = nullptr, n_dec = nullptr,
+                  n_scan = nullptr, n_split = nullptr, n_adv = nullptr, n_test = nullptr, n_ev,
+                  n_part;
+  constexpr int kThreads1 = kEvalThreads<1, SourceFn<Src>>;
   ok = ok && kernel(body, nullptr, (const void*)k_loop_bind<Src>, 1, 32, a_bind, &n_bind);
   cudaGraph_t arms[3] = {nullptr, nullptr, nullptr};
   if (ok) {
@@ -995,11 +1019,13 @@ Workspace::LoopEntry* loop_graph(Workspace& ws, int sms) {
     if (ok)
       for (int i = 0; i < 3; ++i) arms[i] = cp.conditional.phGraph_out[i];
   }
-  ok = ok && kernel(arms[0], nullptr, (const void*)k_loop_eval<N, 1, Src>, sms * 32, 256, a_eval, &n_ev);
+  ok = ok && kernel(arms[0], nullptr, (const void*)k_loop_eval<N, 1, Src>, sms * 32, kThreads1, a_eval, &n_ev);
   ok = ok && kernel(arms[1], nullptr, (const void*)k_loop_eval<N, 8, Src>, sms * 16, 256, a_eval, &n_ev);
+  ok = ok && kernel(arms[1], &n_ev, (const void*)k_loop_partials<Src>, sms * 16, 256, a_la, &n_part);
   ok = ok && kernel(arms[2], nullptr, (const void*)k_loop_eval<N, 32, Src>, sms * 8, 256, a_eval, &n_ev);
-  ok = ok && kernel(body, &n_sw, (const void*)k_loop_partials<Src>, sms * 16, 256, a_la, &n_part);
-  ok = ok && kernel(body, &n_part, (const void*)k_loop_decide<Src>, sms * 16, 256, a_la, &n_dec);
+  ok = ok && kernel(arms[2], &n_ev, (const void*)k_loop_partials<Src>, sms * 16, 256, a_la, &n_part);
+  ok = ok && kernel(body, &n_sw, (const void*)k_loop_tiles<Src>, sms * 4, 128, a_la, &n_tile);
+  ok = ok && kernel(body, &n_tile, (const void*)k_loop_decide<Src>, sms * 16, 256, a_la, &n_dec);
   ok = ok && kernel(body, &n_dec, (const void*)k_loop_scan<Src>, 1, 32, a_la, &n_scan);
   ok = ok && kernel(body, &n_scan, (const void*)k_loop_split<N, Src>, sms * 16, 256, a_la, &n_split);
   ok = ok && kernel(body, &n_split, (const void*)k_loop_advance<Src>, sms, 256, a_la, &n_adv);
@@ -1270,8 +1296,9 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
       const int hb_p = pblocks > 0 ? pmax : 0;
       const int hb_r = rblocks > 0 ? rmax : 0;
       la.hand_back = std::max(hb_p, hb_r);
-      la.k1_min = sms * 512;
-      la.k8_min = sms * 64;
+      const EvalLanes el = eval_lanes<Src>(sms);
+      la.k1_min = el.k1_min;
+      la.k8_min = el.k8_min;
       la.forced_lanes = opt.lanes > 0 ? opt.lanes : 0;
       if (!ws.ck(cudaMemcpyAsync(loop->dargs, loop->hargs, sizeof(la), cudaMemcpyHostToDevice, s)) ||
           !ws.ck(cudaGraphLaunch(loop->exec, s)) ||
@@ -1284,7 +1311,7 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
       st.iterations += la.iterations;
       st.eval_launches += la.iterations;
       st.regions_evaluated += (long long)la.regions;
-      st.launches += 8ll * la.iterations;  // bind, rule, partials, decide, scan, split, advance, test
+      st.launches += 8ll * la.iterations;  // bind, rule, tiles, decide, scan, split, advance, test
       st.device_loops += 1;
       ws.peak_need = std::max(ws.peak_need, la.peak_need);
       c0.iters_done = ws.ctl_host_->iters_done;
@@ -1299,7 +1326,12 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
       continue;
     }
     int K = opt.lanes;
-    if (K <= 0) K = n_cur >= (long long)sms * 512 ? 1 : (n_cur >= (long long)sms * 64 ? 8 : 32);
+    if (K <= 0) {
+      const EvalLanes el = eval_lanes<Src>(sms);
+      K = n_cur >= el.k1_min ? 1 : (n_cur >= el.k8_min ? 8 : 32);
+    }
+    // one lane per region leaves the chunk partials itself
+    const bool partials = Hook::kActive || (K != 1);
     if (ws.timing) ws.ck(cudaEventRecord(ws.ev[0], s));
     if constexpr (Hook::kActive) {
       const int hr = hook.eval(a, n_cur, s);
@@ -1317,13 +1349,16 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
     const long long nchunk = (n_cur + 31) / 32;
     const unsigned pb =
         (unsigned)std::max<long long>(1, std::min<long long>((nchunk + 7) / 8, sms * 16ll));
-    k_partials<<<pb, 256, 0, s>>>(a);
+    if (partials) k_partials<<<pb, 256, 0, s>>>(a);
+    const long long nblk = n_cur / (32 * kTileChunks);
+    if (nblk > 0)
+      k_tiles<<<(unsigned)std::min<long long>((nblk + 3) / 4, sms * 4ll), 128, 0, s>>>(a);
     const unsigned db = (unsigned)std::max(1, std::min((nint + 7) / 8, sms * 16));
     k_decide<<<db, 256, 0, s>>>(a);
     k_scan<<<1, 32, 0, s>>>(a);
     k_split<N><<<pb, 256, 0, s>>>(a);
     k_advance<<<(unsigned)std::max(1, std::min((nint + 255) / 256, sms)), 256, 0, s>>>(a);
-    st.launches += 6;
+    st.launches += 5 + (partials ? 1 : 0) + (nblk > 0 ? 1 : 0);
     if (!ws.ck(cudaMemcpyAsync(ws.ctl_host_, ws.ctl, sizeof(Control), cudaMemcpyDeviceToHost, s)))
       return kErrCuda;
     if (!ws.ck(cudaStreamSynchronize(s))) return kErrCuda;

@@ -27,6 +27,8 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
+#include <utility>
 
 #include "integrands.cuh"
 #include "region_rule.cuh"
@@ -69,6 +71,16 @@ struct ChunkPartial {
   double fin_avg, fin_err;  // finished regions only
   int nactive;
   unsigned mask;  // bit i: slot 32c + i stays active
+};
+
+// Sums of kTileChunks consecutive chunks of one integral (its chunks
+// kTileChunks t .. kTileChunks t + kTileChunks - 1, counted from the
+// start of its segment).
+constexpr int kTileChunks = 256;
+struct TileSum {
+  double sum_avg, sum_err, fin_avg, fin_err;
+  int nactive;
+  int base;  // active regions of the integral before the tile
 };
 
 // List sizes after one iteration's scan.
@@ -138,6 +150,7 @@ struct EngineArgs {
   // chunk partials / prefix / arrival counters
   ChunkPartial* part;
   int* chunk_excl;
+  TileSum* tile;    // multi-launch driver: sums of whole tiles; else null
   unsigned* cmask;  // active bit mask per chunk (optional)
   unsigned* chunk_cnt;
   unsigned* int_cnt;
@@ -172,6 +185,13 @@ template <class F>
 struct SingleSource {
   F f;
   __device__ __forceinline__ const F& get(int) const { return f; }
+};
+
+// Functor F's axis parameters read from a parameter block as they are used.
+template <class F>
+struct ParamView {
+  const GenzParams& p;
+  __device__ __forceinline__ auto axis(int i) const { return F::axis_of(p, i); }
 };
 
 template <class F>
@@ -237,12 +257,29 @@ __device__ __forceinline__ void eval_slot(const Src& src, const RuleTables& T,
   }
 }
 
-// A warp sums the 32 slots of chunk c into a.part[c].
-__device__ __forceinline__ void chunk_partial_warp(const EngineArgs& a, long long c, int lane) {
-  const long long i = c * 32 + lane;
-  const bool valid = i < a.n && a.rid[i] >= 0;
-  const double av = valid ? a.avg[i] : 0.0, er = valid ? a.err[i] : 0.0;
-  const bool act = valid && a.active[i];
+// The integrand type of a source.
+template <class Src>
+using SourceFn = std::decay_t<decltype(std::declval<const Src&>().get(0))>;
+
+// What the thread-per-region evaluator reads integral k's integrand from:
+// a view of its parameter block for axis products of a batch, else the
+// functor.
+template <class Src>
+__device__ __forceinline__ decltype(auto) source_view(const Src& src, int k) {
+  return src.get(k);
+}
+template <class F>
+__device__ __forceinline__ auto source_view(const ParamSource<F>& src, int k) {
+  if constexpr (AxisProductTrait<F>::value)
+    return ParamView<F>{src.params[k]};
+  else
+    return src.get(k);
+}
+
+// Chunk c's partial from its 32 lanes' values (a padding slot holds zeros
+// and is not active); lane 0 stores it.
+__device__ __forceinline__ void store_chunk(const EngineArgs& a, long long c, int lane, double av,
+                                            double er, bool act) {
   double s0 = av, s1 = er, s2 = act ? 0.0 : av, s3 = act ? 0.0 : er;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -262,6 +299,103 @@ __device__ __forceinline__ void chunk_partial_warp(const EngineArgs& a, long lon
     p.mask = b;
     a.part[c] = p;
     if (a.cmask) a.cmask[c] = b;
+  }
+}
+
+// One thread per region: a warp evaluates the 32 slots of chunk c and sums
+// them on the spot, so values and errors never go through memory (24 B a
+// region written and read back by a pass of its own before); only the split
+// axes are stored, beside the chunk's partial.
+template <int N, class Src>
+__device__ __forceinline__ void eval_chunk_warp(const Src& src, const RuleTables& T,
+                                                const EngineArgs& a, long long c, int lane,
+                                                const ItemTable<N>& tab) {
+  const long long slot = c * 32 + lane;
+  const int k = a.rid[slot];
+  double av = 0, er = 0;
+  bool act = false;
+  if (k >= 0) {
+    RegionSums rs;
+    double jac;
+    const ListBox box{a.lo + slot, a.len + slot, a.cap};
+    const auto& f = source_view(src, k);
+    thread_sums<N, SourceFn<Src>>(f, box, tab, T.ratio, rs, jac);
+    const RegionResult r = finish_region<N>(rs, T, jac, 0);
+    av = r.avg;
+    er = r.err;
+    act = er / max_err(av, a.ist[k].epsrel, a.ist[k].epsabs) > 1;
+    a.axis[slot] = r.axis;
+  }
+  __syncwarp();
+  store_chunk(a, c, lane, av, er, act);
+}
+
+// A warp sums the 32 slots of chunk c into a.part[c].
+__device__ __forceinline__ void chunk_partial_warp(const EngineArgs& a, long long c, int lane) {
+  const long long i = c * 32 + lane;
+  const bool valid = i < a.n && a.rid[i] >= 0;
+  const double av = valid ? a.avg[i] : 0.0, er = valid ? a.err[i] : 0.0;
+  const bool act = valid && a.active[i];
+  store_chunk(a, c, lane, av, er, act);
+}
+
+// A warp sums the whole tile (if any) that starts within the absolute
+// chunks [kTileChunks w, kTileChunks (w + 1)): a.tile[w], and the active
+// counts before each of its chunks, from the tile's start, to chunk_excl.
+// Such a tile's integral owns the last chunk of that range, so there is one
+// at most.  Tiles are counted from the segment's start, so an integral's
+// sums do not depend on where its segment lies.
+__device__ __forceinline__ void tile_sum_warp(const EngineArgs& a, long long w, int lane) {
+  constexpr int kPer = kTileChunks / 32;
+  const int k = a.rid[(kTileChunks * w + kTileChunks - 1) * 32];
+  const int c0 = a.ist[k].seg_start / 32, nc = (a.ist[k].seg_count + 31) / 32;
+  const long long t = w - c0 / kTileChunks;
+  if (t < 0 || kTileChunks * (t + 1) > nc) return;
+  const long long s = c0 + kTileChunks * t;
+  double v0[kPer], v1[kPer], v2[kPer], v3[kPer];
+  int na[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const ChunkPartial& p = a.part[s + 32 * i + lane];
+    v0[i] = p.sum_avg;
+    v1[i] = p.sum_err;
+    v2[i] = p.fin_avg;
+    v3[i] = p.fin_err;
+    na[i] = p.nactive;
+  }
+  double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+  int run = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    s0 += v0[i];
+    s1 += v1[i];
+    s2 += v2[i];
+    s3 += v3[i];
+    int incl = na[i];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += u;
+    }
+    a.chunk_excl[s + 32 * i + lane] = run + incl - na[i];
+    run += __shfl_sync(0xffffffffu, incl, 31);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, off);
+    s3 += __shfl_xor_sync(0xffffffffu, s3, off);
+  }
+  if (lane == 0) {
+    TileSum o;
+    o.sum_avg = s0;
+    o.sum_err = s1;
+    o.fin_avg = s2;
+    o.fin_err = s3;
+    o.nactive = run;
+    o.base = 0;
+    a.tile[w] = o;
   }
 }
 
@@ -318,7 +452,11 @@ __device__ __forceinline__ void decide_integral(IntegralState& is, double s0, do
 
 // A warp combines integral k's chunk partials, writes the exclusive scan
 // of active counts over its chunks, and takes the stop decision
-// (GPUKernelquad.cu:565-605).
+// (GPUKernelquad.cu:565-605).  With tiles (a.tile), whole tiles of the
+// integral come summed already (tile_sum_warp) and only the chunks after
+// the last one are read: one warp walking every chunk took 4 ms for the
+// 130 k chunks of a 4 M region integral, a fifth of the time of a batch
+// that has one such integral.
 __device__ __forceinline__ void decide_warp(const EngineArgs& a, int k, int lane) {
   IntegralState& is = a.ist[k];
   if (is.state != kStateRunning) {
@@ -330,8 +468,17 @@ __device__ __forceinline__ void decide_warp(const EngineArgs& a, int k, int lane
   }
   const int c0 = is.seg_start / 32;
   const int nc = (is.seg_count + 31) / 32;
+  const int nt = a.tile ? nc / kTileChunks : 0;
+  TileSum* tile = a.tile + (nt ? c0 / kTileChunks : 0);
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-  for (int c = lane; c < nc; c += 32) {
+  for (int t = lane; t < nt; t += 32) {
+    const TileSum p = tile[t];
+    s0 += p.sum_avg;
+    s1 += p.sum_err;
+    s2 += p.fin_avg;
+    s3 += p.fin_err;
+  }
+  for (int c = nt * kTileChunks + lane; c < nc; c += 32) {
     const ChunkPartial p = a.part[c0 + c];
     s0 += p.sum_avg;
     s1 += p.sum_err;
@@ -346,7 +493,19 @@ __device__ __forceinline__ void decide_warp(const EngineArgs& a, int k, int lane
     s3 += __shfl_xor_sync(0xffffffffu, s3, off);
   }
   int running = 0;
-  for (int base = 0; base < nc; base += 32) {
+  for (int base = 0; base < nt; base += 32) {
+    const int t = base + lane;
+    const int v = t < nt ? tile[t].nactive : 0;
+    int incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += u;
+    }
+    if (t < nt) tile[t].base = running + incl - v;
+    running += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  for (int base = nt * kTileChunks; base < nc; base += 32) {
     const int c = base + lane;
     const int v = c < nc ? a.part[c0 + c].nactive : 0;
     int incl = v;
@@ -413,55 +572,51 @@ __device__ __forceinline__ void scan_warp(const EngineArgs& a, int n_left_in, It
 // integrals) or the leftover list (integrals just handed to phase 2).
 template <int N>
 __device__ __forceinline__ void split_chunk_warp(const EngineArgs& a, long long c, int lane) {
+  const ChunkPartial* part = a.part + c;
+  const unsigned b = part->mask;
+  if (!b) return;
+  // a chunk belongs to one integral, and its first slot is never padding
+  const int k = a.rid[c * 32];
+  const IntegralState& is = a.ist[k];
+  const int state = is.state;
+  const bool next = state == kStateRunning && is.next_count > 0;
+  if (!next && !(state == kStatePhase2 && is.left_new > 0)) return;
+  if (!((b >> lane) & 1u)) return;
   const long long i = c * 32 + lane;
-  const int k = i < a.n ? a.rid[i] : -1;
-  bool act = k >= 0 && a.active[i];
-  int state = kStateDone;
-  if (act) {
-    state = a.ist[k].state;
-    act = (state == kStateRunning && a.ist[k].next_count > 0) ||
-          (state == kStatePhase2 && a.ist[k].left_new > 0);
-  }
-  const unsigned b = __ballot_sync(0xffffffffu, act);
-  if (!act) return;
-  const int rank = a.chunk_excl[c] + __popc(b & ((1u << lane) - 1u));
+  int rank = a.chunk_excl[c] + __popc(b & ((1u << lane) - 1u));
+  const int c0 = is.seg_start / 32, nt = (is.seg_count + 31) / 32 / kTileChunks;
+  const int t = (int)(c - c0) / kTileChunks;
+  if (t < nt) rank += a.tile[c0 / kTileChunks + t].base;
   const int ax = a.axis[i];
   double* dlo;
   double* dlen;
   int* drid;
   long long dcap, dst;
-  if (state == kStatePhase2) {
+  if (!next) {
     dlo = a.left_lo;
     dlen = a.left_len;
     drid = a.left_rid;
     dcap = a.left_cap;
-    dst = a.ist[k].left_start + 2ll * rank;
+    dst = is.left_start + 2ll * rank;
   } else {
     dlo = a.nlo;
     dlen = a.nlen;
     drid = a.nrid;
     dcap = a.ncap;
-    dst = a.ist[k].next_start + 2ll * rank;
+    dst = is.next_start + 2ll * rank;
   }
+  // dst and the capacities are even: the children of a region are stored as
+  // one 16-byte pair per axis
 #pragma unroll
   for (int d = 0; d < N; ++d) {
     const double l = a.lo[(long long)d * a.cap + i];
     const double w = a.len[(long long)d * a.cap + i];
-    if (d == ax) {
-      const double h = w / 2;
-      dlo[(long long)d * dcap + dst] = l;
-      dlo[(long long)d * dcap + dst + 1] = l + 1 * h;
-      dlen[(long long)d * dcap + dst] = h;
-      dlen[(long long)d * dcap + dst + 1] = h;
-    } else {
-      dlo[(long long)d * dcap + dst] = l;
-      dlo[(long long)d * dcap + dst + 1] = l;
-      dlen[(long long)d * dcap + dst] = w;
-      dlen[(long long)d * dcap + dst + 1] = w;
-    }
+    const double h = d == ax ? w / 2 : w;
+    *reinterpret_cast<double2*>(dlo + (long long)d * dcap + dst) =
+        make_double2(l, d == ax ? l + 1 * h : l);
+    *reinterpret_cast<double2*>(dlen + (long long)d * dcap + dst) = make_double2(h, h);
   }
-  drid[dst] = k;
-  drid[dst + 1] = k;
+  *reinterpret_cast<int2*>(drid + dst) = make_int2(k, k);
 }
 
 // Padding ids of integral k's next segment, and the segment hand-over
@@ -486,23 +641,46 @@ __device__ __forceinline__ void finish_integral(const EngineArgs& a, int k) {
 // ---------------------------------------------------------------------------
 // Multi-launch driver kernels (one launch per step).
 // ---------------------------------------------------------------------------
+// Threads of a block of the rule kernel with K lanes per region, and blocks
+// per SM.  Point by point: two blocks of 256 (at most 128 registers); the
+// kernel is bound by FP64 latency, so warps in flight matter more than a few
+// spilled values.
+template <int K, class F>
+constexpr int kEvalThreads = K == 1 && detail::kFactored<F> ? 128 : 256;
+template <int K, class F>
+constexpr int kEvalMinBlocks = K == 1 && detail::kFactored<F> ? 4 : 2;
+
 template <int N, int K, class Src>
-// Two blocks per SM (at most 128 registers): the rule kernel is bound by
-// FP64 latency, so warps in flight matter more than a few spilled values.
-#ifndef CUB_EVAL_MIN_BLOCKS
-#define CUB_EVAL_MIN_BLOCKS 2
-#endif
-__global__ void __launch_bounds__(256, CUB_EVAL_MIN_BLOCKS) k_eval(Src src, RuleTables T, EngineArgs a) {
+__device__ __forceinline__ void eval_list(const Src& src, const RuleTables& T, const EngineArgs& a,
+                                          const detail::ItemTable<N>& tab) {
+  const int lane = threadIdx.x % (K == 1 ? 32 : K);
+  if constexpr (K == 1) {
+    const long long nchunk = a.n / 32, nwarp = (long long)gridDim.x * (blockDim.x / 32);
+    for (long long c = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; c < nchunk;
+         c += nwarp)
+      detail::eval_chunk_warp<N>(src, T, a, c, lane, tab);
+  } else {
+    constexpr int kGroups = 256 / K;
+    const unsigned gmask =
+        (K == 32) ? 0xffffffffu : (((1u << (K & 31)) - 1u) << ((threadIdx.x & 31) & ~(K - 1)));
+    for (long long slot = (long long)blockIdx.x * kGroups + threadIdx.x / K; slot < a.n;
+         slot += (long long)gridDim.x * kGroups)
+      detail::eval_slot<N, K>(src, T, a, slot, lane, gmask, tab);
+  }
+}
+
+// The rule over the current list.  K = 1 also leaves the chunk partials;
+// K = 8 and 32 need k_partials after them.
+template <int N, int K, class Src>
+__global__ void __launch_bounds__((kEvalThreads<K, detail::SourceFn<Src>>),
+                                  (kEvalMinBlocks<K, detail::SourceFn<Src>>))
+    k_eval(Src src, RuleTables T, EngineArgs a) {
   __shared__ detail::ItemTable<N> tab;
-  if (threadIdx.x == 0) tab.fill();
-  __syncthreads();
-  constexpr int kGroups = 256 / K;
-  const int lane = threadIdx.x % K;
-  const unsigned gmask =
-      (K == 32) ? 0xffffffffu : (((1u << K) - 1u) << ((threadIdx.x & 31) & ~(K - 1)));
-  for (long long slot = (long long)blockIdx.x * kGroups + threadIdx.x / K; slot < a.n;
-       slot += (long long)gridDim.x * kGroups)
-    detail::eval_slot<N, K>(src, T, a, slot, lane, gmask, tab);
+  if (!(K == 1 && detail::kFactored<detail::SourceFn<Src>>)) {
+    if (threadIdx.x == 0) tab.fill();
+    __syncthreads();
+  }
+  eval_list<N, K>(src, T, a, tab);
 }
 
 static __global__ void __launch_bounds__(256) k_partials(EngineArgs a) {
@@ -510,6 +688,13 @@ static __global__ void __launch_bounds__(256) k_partials(EngineArgs a) {
   for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; c < nchunk;
        c += (long long)gridDim.x * blockDim.x / 32)
     detail::chunk_partial_warp(a, c, threadIdx.x & 31);
+}
+
+static __global__ void __launch_bounds__(128) k_tiles(EngineArgs a) {
+  const long long nw = a.n / (32 * kTileChunks);
+  for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw;
+       w += (long long)gridDim.x * blockDim.x / 32)
+    detail::tile_sum_warp(a, w, threadIdx.x & 31);
 }
 
 static __global__ void __launch_bounds__(256) k_decide(EngineArgs a) {

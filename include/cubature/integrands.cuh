@@ -8,6 +8,21 @@
 //
 // Parameters travel as GenzParams (one per integral); load() turns them
 // into the functor's register form, folding constant work (a^2, a^-2).
+//
+// Axis products.  A functor whose value is a product of one factor per axis
+// (Gaussian, product peak) says so with kAxisProduct, and the
+// thread-per-region evaluator (axis_product_sums, region_rule.cuh) then
+// forms the rule's set sums from per-axis factors.  It provides
+//   axis(i)         axis i's parameters (also from a parameter block,
+//                   axis_of), whose term(x) is what the axis contributes at x,
+//   start(), step(acc, t), finish(acc)   the value as a left-to-right fold
+//                   of the terms: operator() is that fold, so values formed
+//                   either way have the same bits,
+//   factor(t)       the axis' factor of the value,
+//   factor2(t, s)   factor(t) + factor(s),
+//   over(v, t)      v / factor(t),
+//   kNoise          a bound of the relative rounding error of the fold's
+//                   value and of the factors, with room to spare.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,14 +58,36 @@ struct Gaussian {
     for (int i = 0; i < N; ++i) { g.a[i] = p.a[i]; g.u[i] = p.u[i]; }
     return g;
   }
+  static constexpr bool kAxisProduct = true;
+  struct Axis {
+    double a, u;
+    __device__ __forceinline__ double term(double x) const { return a * (x - u); }
+  };
+  __device__ __forceinline__ static Axis axis_of(const GenzParams& p, int i) {
+    return {p.a[i], p.u[i]};
+  }
+  __device__ __forceinline__ Axis axis(int i) const { return {a[i], u[i]}; }
+  __device__ __forceinline__ static double start() { return 0.0; }
+  __device__ __forceinline__ static double step(double s, double t) { return fma(t, t, s); }
+  __device__ __forceinline__ static double finish(double s) { return exp(-s); }
+  // exp(-t^2) with the rounding of t^2 corrected: a factor's error enters
+  // many points alike, and does not average out as the points' own do
+  __device__ __forceinline__ static double factor(double t) {
+    const double tt = t * t;
+    const double y = exp(-tt);
+    return y > 0 ? fma(-fma(t, t, -tt), y, y) : y;
+  }
+  __device__ __forceinline__ static double factor2(double t, double s) {
+    return factor(t) + factor(s);
+  }
+  __device__ __forceinline__ static double over(double v, double t) { return v / exp(-(t * t)); }
+  // the exponent is at most 745 where the value is not zero, summed in N steps
+  static constexpr double kNoise = 2e-13 * N;
   __device__ __forceinline__ double operator()(const double* x) const {
-    double s = 0;
+    double s = start();
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const double t = a[i] * (x[i] - u[i]);
-      s += t * t;
-    }
-    return exp(-s);
+    for (int i = 0; i < N; ++i) s = step(s, axis(i).term(x[i]));
+    return finish(s);
   }
 };
 
@@ -104,14 +141,44 @@ struct ProductPeak {
     for (int i = 0; i < N; ++i) { q.ia2[i] = 1 / (p.a[i] * p.a[i]); q.u[i] = p.u[i]; }
     return q;
   }
-  __device__ __forceinline__ double operator()(const double* x) const {
-    double den = 1;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const double t = x[i] - u[i];
-      den *= ia2[i] + t * t;
+  static constexpr bool kAxisProduct = true;
+  struct Axis {
+    double ia2, u;
+    __device__ __forceinline__ double term(double x) const {
+      const double t = x - u;
+      return fma(t, t, ia2);
     }
-    return 1 / den;
+  };
+  __device__ __forceinline__ static Axis axis_of(const GenzParams& p, int i) {
+    return {1 / (p.a[i] * p.a[i]), p.u[i]};
+  }
+  __device__ __forceinline__ Axis axis(int i) const { return {ia2[i], u[i]}; }
+  __device__ __forceinline__ static double start() { return 1.0; }
+  __device__ __forceinline__ static double step(double den, double q) { return den * q; }
+  __device__ __forceinline__ static double finish(double den) { return 1 / den; }
+  __device__ __forceinline__ static double factor(double q) { return 1 / q; }
+  // 1/q + 1/p as (q + p) / (q p) with the roundings of the sum, the product
+  // and the quotient corrected (a factor's error enters many points alike);
+  // two divisions where the product leaves the normal range (a double's
+  // biased exponent is in its high word's top bits)
+  __device__ __forceinline__ static double factor2(double q, double p) {
+    const double qp = q * p;
+    const unsigned e = (unsigned)__double2hiint(qp) >> 20;
+    if (e - 128u < 1791u) {
+      const double s = q + p, b = s - q;
+      const double es = (q - (s - b)) + (p - b), ep = fma(q, p, -qp);
+      const double r = __drcp_rn(qp), y = s * r;
+      return fma(fma(-y, ep, fma(-y, qp, s) + es), r, y);
+    }
+    return 1 / q + 1 / p;
+  }
+  __device__ __forceinline__ static double over(double v, double q) { return v * q; }
+  static constexpr double kNoise = 4e-15 * (N + 6);
+  __device__ __forceinline__ double operator()(const double* x) const {
+    double den = start();
+#pragma unroll
+    for (int i = 0; i < N; ++i) den = step(den, axis(i).term(x[i]));
+    return finish(den);
   }
 };
 

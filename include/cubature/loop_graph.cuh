@@ -10,8 +10,9 @@
 //
 //   bind     reads the list length and buffer parity from the control block,
 //            binds the iteration's arguments and picks the rule kernel's
-//            lanes per region (a SWITCH node over three k_eval variants);
-//   eval, partials, decide, scan, split, advance
+//            lanes per region (a SWITCH node over three k_eval variants;
+//            those with several lanes per region are followed by partials);
+//   eval, tiles, decide, scan, split, advance
 //            the multi-launch kernels, reading their arguments from device
 //            memory instead of launch parameters;
 //   test     continues while integrals are running, the next list fits the
@@ -49,7 +50,7 @@ struct LoopArgs {
 };
 
 // Lanes per region of the multi-launch rule kernel for a list of n slots
-// (0, 1, 2: 1, 8, 32 lanes).
+// (0, 1, 2: 1, 8, 32 lanes); k1_min and k8_min come from eval_lanes.
 template <class Src>
 __device__ __forceinline__ int loop_lane_case(const LoopArgs<Src>& la, long long n) {
   const int k = la.forced_lanes ? la.forced_lanes : (n >= la.k1_min ? 1 : (n >= la.k8_min ? 8 : 32));
@@ -101,22 +102,17 @@ __device__ __forceinline__ void loop_load(const LoopArgs<Src>* la, LoopShared<Sr
 // as k_eval does; from shared memory the one-lane-per-region variant
 // spilled.  Blocks beyond the list's end leave before loading anything.
 template <int N, int K, class Src>
-__global__ void __launch_bounds__(256, CUB_EVAL_MIN_BLOCKS) k_loop_eval(const LoopArgs<Src>* la,
-                                                                        RuleTables T) {
-  constexpr int kGroups = 256 / K;
+__global__ void __launch_bounds__((kEvalThreads<K, detail::SourceFn<Src>>),
+                                  (kEvalMinBlocks<K, detail::SourceFn<Src>>))
+    k_loop_eval(const LoopArgs<Src>* la, RuleTables T) {
+  constexpr int kGroups = kEvalThreads<K, detail::SourceFn<Src>> / K;
   if ((long long)blockIdx.x * kGroups >= la->it.n) return;
   __shared__ detail::ItemTable<N> tab;
   __shared__ LoopShared<Src> sh;
-  if (threadIdx.x == 0) tab.fill();
+  if (!(K == 1 && detail::kFactored<detail::SourceFn<Src>>) && threadIdx.x == 0) tab.fill();
   loop_load(la, sh);
   __syncthreads();
-  const int lane = threadIdx.x % K;
-  const unsigned gmask =
-      (K == 32) ? 0xffffffffu : (((1u << K) - 1u) << ((threadIdx.x & 31) & ~(K - 1)));
-  const EngineArgs& a = sh.a;
-  for (long long slot = (long long)blockIdx.x * kGroups + threadIdx.x / K; slot < a.n;
-       slot += (long long)gridDim.x * kGroups)
-    detail::eval_slot<N, K>(sh.src, T, a, slot, lane, gmask, tab);
+  eval_list<N, K>(sh.src, T, sh.a, tab);
 }
 
 template <class Src>
@@ -126,6 +122,15 @@ __global__ void __launch_bounds__(256) k_loop_partials(const LoopArgs<Src>* la) 
   for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; c < nchunk;
        c += (long long)gridDim.x * blockDim.x / 32)
     detail::chunk_partial_warp(a, c, threadIdx.x & 31);
+}
+
+template <class Src>
+__global__ void __launch_bounds__(128) k_loop_tiles(const LoopArgs<Src>* la) {
+  const EngineArgs a = la->it;
+  const long long nw = a.n / (32 * kTileChunks);
+  for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; w < nw;
+       w += (long long)gridDim.x * blockDim.x / 32)
+    detail::tile_sum_warp(a, w, threadIdx.x & 31);
 }
 
 template <class Src>

@@ -7,10 +7,17 @@
 
 namespace cubature {
 
+// List length from which k_step_rule takes one thread per region (below: a
+// warp).  Point by point: when the list fills the chip.
+template <class F>
+inline long long rule_thread_min(int sms) {
+  return detail::kFactored<F> ? 0 : sms * 512ll;
+}
+
 // Rule + classification over one integral's SoA list (INTEGRATE_GPU_PHASE1,
 // GPUQuadPhases.cu:38-79).
 template <int N, int K, class F>
-__global__ void __launch_bounds__(256) k_step_rule(F f, RuleTables T, long long n,
+__global__ void __launch_bounds__((K == 1 && detail::kFactored<F>) ? 128 : 256) k_step_rule(F f, RuleTables T, long long n,
                                                    const double* lo, const double* len,
                                                    long long ld, double epsrel, double epsabs,
                                                    double* avg, double* err, int* axis,
@@ -18,25 +25,30 @@ __global__ void __launch_bounds__(256) k_step_rule(F f, RuleTables T, long long 
   __shared__ detail::ItemTable<N> tab;
   if (threadIdx.x == 0) tab.fill();
   __syncthreads();
-  constexpr int kGroups = 256 / K;
+  const int kGroups = (int)blockDim.x / K;
   const int lane = threadIdx.x % K;
   const unsigned gmask =
       (K == 32) ? 0xffffffffu : (((1u << K) - 1u) << ((threadIdx.x & 31) & ~(K - 1)));
   for (long long i = (long long)blockIdx.x * kGroups + threadIdx.x / K; i < n;
        i += (long long)gridDim.x * kGroups) {
-    double L[N], H[N];
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      L[d] = lo[(long long)d * ld + i];
-      H[d] = len[(long long)d * ld + i];
-    }
     detail::RegionSums rs;
-    detail::region_point_sums<N, K>(f, L, H, lane, tab, T.ratio, rs);
-    if (K > 1) detail::reduce_lanes<K>(rs, gmask);
-    if (lane == 0) {
-      double jac = 1;
+    double jac;
+    if constexpr (K == 1) {
+      detail::thread_sums<N, F>(f, detail::ListBox{lo + i, len + i, ld}, tab, T.ratio, rs, jac);
+    } else {
+      double L[N], H[N];
+#pragma unroll
+      for (int d = 0; d < N; ++d) {
+        L[d] = lo[(long long)d * ld + i];
+        H[d] = len[(long long)d * ld + i];
+      }
+      detail::region_point_sums<N, K>(f, L, H, lane, tab, T.ratio, rs);
+      detail::reduce_lanes<K>(rs, gmask);
+      jac = 1;
 #pragma unroll
       for (int d = 0; d < N; ++d) jac = __dmul_rn(jac, H[d]);
+    }
+    if (lane == 0) {
       const detail::RegionResult r = detail::finish_region<N>(rs, T, jac, 0);
       avg[i] = r.avg;
       err[i] = r.err;

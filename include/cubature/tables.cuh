@@ -139,10 +139,12 @@ struct Table7 {
   double inv2s2;  // 1 / (2 sigma^2)
   double offset;
 
+  __device__ __forceinline__ double kernel_arg(double x3, double x4, double x5, double x6) const {
+    return fma(4.0, x3, -fma(0.1, x5 + x6, fma(2.0, x4, offset)));
+  }
+  __device__ __forceinline__ double kernel(double r) const { return exp(-r * r * inv2s2); }
   __device__ __forceinline__ double operator()(const double* x) const {
-    const double mu = offset + 2.0 * x[4] + 0.1 * (x[5] + x[6]);
-    const double r = 4.0 * x[3] - mu;
-    return spline(x[0]) * grid(x[1], x[2]) * exp(-r * r * inv2s2);
+    return spline(x[0]) * grid(x[1], x[2]) * kernel(kernel_arg(x[3], x[4], x[5], x[6]));
   }
 };
 

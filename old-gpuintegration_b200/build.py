@@ -50,7 +50,7 @@ def _deps() -> list[Path]:
 
 
 # headers that one source alone includes
-ONLY = {"mlp.cuh": "mlp.cu", "umma.cuh": "mlp.cu"}
+ONLY = {"mlp.cuh": "mlp.cu", "umma.cuh": "mlp.cu", "table_sums.cuh": "capi_tables.cu"}
 
 
 def _stale(obj: Path, src: Path, deps: list[Path]) -> bool:

@@ -57,8 +57,8 @@ int FamilyDim<N, Fam>::rule(const GenzParams& p, long long n, const double* lo, 
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = sm_count(dev);
-  if (n >= (long long)sms * 512) {
-    constexpr int kThreads = 256;
+  if (n >= rule_thread_min<Fam<N>>(sms)) {
+    constexpr int kThreads = detail::kFactored<Fam<N>> ? 128 : 256;
     const long long blocks =
         std::min<long long>((n + kThreads - 1) / kThreads, (long long)sms * 32);
     k_step_rule<N, 1><<<(unsigned)blocks, kThreads, 0, s>>>(f, T, n, lo, len, ld, epsrel, epsabs,

@@ -7,7 +7,7 @@
 #include <vector>
 
 #include "capi_internal.h"
-#include "cubature/tables.cuh"
+#include "cubature/table_sums.cuh"
 
 using namespace cubature;
 using namespace cubature::capi;
