@@ -1046,6 +1046,90 @@ Workspace::LoopEntry* loop_graph(Workspace& ws, int sms) {
 
 }  // namespace detail
 
+// Launch shape and memory of the second phase over `boxes` boxes.
+template <int N, class Src>
+struct Phase2Launch {
+  static constexpr bool kSplit = detail::AxisProductTrait<detail::SourceFn<Src>>::value;
+  long long blocks = 1;
+  bool smem_heap = false;
+  size_t heap_smem = 0;
+
+  bool wide = false;
+
+  bool reserve(Workspace& ws, const Options& opt, long long boxes, int sms) {
+    int per_sm = 0;
+    if constexpr (kSplit) {
+      wide = boxes <= kSplitWideBoxes;
+      return wide ? reserve_split<kSplitLanes<N, true>>(ws, opt, boxes, sms)
+                  : reserve_split<kSplitLanes<N, false>>(ws, opt, boxes, sms);
+    } else {
+      // the heaps in shared memory when two blocks of them fit on an SM (the
+      // default 2048 bisections: 98 KB a block), else in the global slab
+      heap_smem = detail::phase2_heap_smem(opt.phase2_max_regions);
+      smem_heap =
+          heap_smem <= 100 * 1024 &&
+          cudaFuncSetAttribute(k_phase2<N, Src, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)heap_smem) == cudaSuccess;
+      if (!smem_heap) cudaGetLastError();
+      if (smem_heap)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase2<N, Src, true>, 128,
+                                                      heap_smem);
+      else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase2<N, Src, false>, 128, 0);
+      blocks = std::min<long long>((long long)sms * std::max(1, per_sm), (boxes + 3) / 4);
+      blocks = std::max<long long>(blocks, 1);
+      const size_t n = (size_t)blocks * 4 * (opt.phase2_max_regions + 2);
+      return ws.reserve_slab(sizeof(P2Region<N>) * n,
+                             smem_heap ? 1 : n * (sizeof(P2HeapEnt) / sizeof(int)));
+    }
+  }
+
+  void run(const Src& src, const RuleTables& T, const Phase2Args& p, cudaStream_t s) const {
+    if constexpr (kSplit) {
+      if (wide)
+        run_split<kSplitLanes<N, true>>(src, T, p, s);
+      else
+        run_split<kSplitLanes<N, false>>(src, T, p, s);
+    } else {
+      if (smem_heap)
+        k_phase2<N, Src, true><<<(unsigned)blocks, 128, heap_smem, s>>>(src, T, p);
+      else
+        k_phase2<N, Src, false><<<(unsigned)blocks, 128, 0, s>>>(src, T, p);
+    }
+  }
+
+ private:
+  template <int K>
+  bool reserve_split(Workspace& ws, const Options& opt, long long boxes, int sms) {
+    // a pool and a heap per box in flight: as many boxes as the chip holds,
+    // fewer when memory is short
+    constexpr int kBoxes = kSplitThreads / (2 * K);  // per block
+    int per_sm = 0;
+    if (!ws.ck(cudaFuncSetAttribute(k_phase2_split<N, K, Src>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSplitSmem<K>)) ||
+        !ws.ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, k_phase2_split<N, K, Src>, kSplitThreads, kSplitSmem<K>)))
+      return false;
+    blocks = std::min<long long>((long long)sms * std::max(1, per_sm),
+                                 (boxes + kBoxes - 1) / kBoxes);
+    const size_t stride = (size_t)split_stride(opt.phase2_max_regions);
+    for (blocks = std::max<long long>(blocks, 1);; blocks /= 2) {
+      const size_t n = (size_t)blocks * kBoxes * stride;
+      if (ws.reserve_slab(sizeof(P2Region<N>) * n, n * (sizeof(P2HeapEnt) / sizeof(int))))
+        return true;
+      cudaGetLastError();
+      if (blocks == 1) return false;
+    }
+  }
+
+  template <int K>
+  void run_split(const Src& src, const RuleTables& T, const Phase2Args& p,
+                 cudaStream_t s) const {
+    k_phase2_split<N, K, Src><<<(unsigned)blocks, kSplitThreads, kSplitSmem<K>, s>>>(src, T, p);
+  }
+};
+
 // Rule evaluation step of the multi-launch driver when the caller supplies
 // its own (NoHook: the engine's k_eval).  A hook's eval(args, n, stream)
 // evaluates the n slots of the current list into args.avg/err/axis/active
@@ -1418,28 +1502,8 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
   if (status == kOk && n_left > 0) {
     // phase 2 on the leftover boxes [box0, box1)
     states_fresh = false;
-    // the heaps in shared memory when two blocks of them fit on an SM (the
-    // default 2048 bisections: 98 KB a block), else in the global slab
-    const size_t heap_smem = detail::phase2_heap_smem(opt.phase2_max_regions);
-    const bool smem_heap =
-        heap_smem <= 100 * 1024 &&
-        cudaFuncSetAttribute(k_phase2<N, Src, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)heap_smem) == cudaSuccess;
-    if (!smem_heap) cudaGetLastError();
-    int dev_blocks = 0;
-    if (smem_heap)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dev_blocks, k_phase2<N, Src, true>, 128,
-                                                    heap_smem);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dev_blocks, k_phase2<N, Src, false>, 128, 0);
-    dev_blocks = std::max(1, dev_blocks);
-    long long blocks = std::min<long long>((long long)sms * dev_blocks, (box1 - box0 + 3) / 4);
-    blocks = std::max<long long>(blocks, 1);
-    const long long nwarps = blocks * 4;
-    const int stride = opt.phase2_max_regions + 2;
-    if (!ws.reserve_slab(sizeof(P2Region<N>) * nwarps * stride,
-                         smem_heap ? 1 : (size_t)nwarps * stride * (sizeof(P2HeapEnt) / sizeof(int))))
-      return kErrCuda;
+    Phase2Launch<N, Src> launch;
+    if (!launch.reserve(ws, opt, box1 - box0, sms)) return kErrCuda;
     if (shard) {
       // boxes of other shares contribute nothing to the collection
       if (!ws.ck(cudaMemsetAsync(ws.left_res, 0, sizeof(LeftoverResult) * n_left, s)))
@@ -1466,10 +1530,7 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
     // one integral's shares follow the reference's leftover order
     p.pair_half = shard && opt.shard_world > 1 && nint == 1 ? (int)(n_left / 2) : 0;
     if (ws.timing) ws.ck(cudaEventRecord(ws.ev[2], s));
-    if (smem_heap)
-      k_phase2<N, Src, true><<<(unsigned)blocks, 128, heap_smem, s>>>(src, T, p);
-    else
-      k_phase2<N, Src, false><<<(unsigned)blocks, 128, 0, s>>>(src, T, p);
+    launch.run(src, T, p, s);
     if (ws.timing) ws.ck(cudaEventRecord(ws.ev[3], s));
     st.phase2_boxes += box1 - box0;
     const unsigned cb = (unsigned)std::max(1, std::min((nint + 7) / 8, sms * 16));

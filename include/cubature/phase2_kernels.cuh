@@ -5,7 +5,9 @@
 // first phase on its own: serial Cuhre with the box's own tolerance
 // (ERR <= max(epsrel |RESULT|, epsabs)) and at most 2048 bisections.
 //
-// Re-design for sm_100a: one warp per leftover box, persistent warps pulling
+// Two kernels.  Integrands that are products over the axes take
+// k_phase2_split, a few lanes per box and several boxes per warp; all others
+// k_phase2: one warp per leftover box, persistent warps pulling
 // boxes from an atomic counter.  Each step bisects the box's exact maximum
 // error subregion (a binary heap kept by lane 0, each entry holding the
 // subregion's error beside its index), and the two children are
@@ -390,6 +392,298 @@ __global__ void __launch_bounds__(128, kShared ? 2 : 3) k_phase2(Src src, RuleTa
       o.nregions = nreg;
       o.failed = failed;
       a.out[box] = o;
+    }
+    __syncwarp();
+  }
+}
+
+namespace detail {
+
+// Binary max-heap of one box, the comparisons of heap_push / heap_pop (same
+// bisection order).  The first kTop entries (eight levels, the whole heap of
+// most boxes) lie in shared memory, the others in global memory: entry i at
+// g[i + 1], so that the two children of an entry share a 32-byte sector.
+// Keys are the bits of the errors, which order as the non-negative errors
+// do (the subregions of a box whose error is not a number are never
+// compared: the box stops at its first bisection).
+//
+// In global memory alone the pop took 3.5 k and the two pushes 2 k of the
+// 10 k cycles of a bisection late in a box of 2048.
+struct SplitHeap {
+  static constexpr int kTop = 255;
+  static constexpr int kBytes = 3072;  // kTop keys and indices
+  unsigned long long* key;
+  int* id;
+  P2HeapEnt* g;
+
+  __device__ __forceinline__ void load(int i, unsigned long long& k, int& x) const {
+    if (i < kTop) {
+      k = key[i];
+      x = id[i];
+    } else {
+      const P2HeapEnt e = g[i + 1];
+      k = (unsigned long long)__double_as_longlong(e.err);
+      x = e.idx;
+    }
+  }
+  __device__ __forceinline__ void store(int i, unsigned long long k, int x) const {
+    if (i < kTop) {
+      key[i] = k;
+      id[i] = x;
+    } else {
+      g[i + 1] = P2HeapEnt{__longlong_as_double((long long)k), x, 0};
+    }
+  }
+  __device__ __forceinline__ void push(int& hn, int idx, double err) const {
+    int i = hn++;
+    const unsigned long long k = (unsigned long long)__double_as_longlong(err);
+    while (i > 0) {
+      const int p = (i - 1) / 2;
+      unsigned long long pk;
+      int px;
+      load(p, pk, px);
+      if (pk >= k) break;
+      store(i, pk, px);
+      i = p;
+    }
+    store(i, k, idx);
+  }
+  __device__ __forceinline__ int pop(int& hn) const {
+    const int top = id[0];
+    unsigned long long k;
+    int x;
+    load(--hn, k, x);
+    int i = 0;
+    // children l and l + 1 lie on the same side of kTop (both odd); entry
+    // l + 1 may be past the end, and is then not used
+    for (int l = 1; l < hn; l = 2 * i + 1) {
+      unsigned long long kl, kr;
+      int xl, xr;
+      load(l, kl, xl);
+      load(l + 1, kr, xr);
+      int m = i, xm = x;
+      unsigned long long km = k;
+      if (kl > km) {
+        m = l;
+        km = kl;
+        xm = xl;
+      }
+      if (l + 1 < hn && kr > km) {
+        m = l + 1;
+        km = kr;
+        xm = xr;
+      }
+      if (m == i) break;
+      store(i, km, xm);
+      i = m;
+    }
+    store(i, k, x);
+    return top;
+  }
+};
+
+// A subregion of a leftover box in the integrand's coordinates: the pool
+// entry `r` (local coordinates), or its child `side` when ax >= 0.
+template <int N>
+struct SubBox {
+  const P2Region<N>* r;
+  const double* bl;  // the leftover box: lower corner and widths, stride ld
+  const double* bw;
+  long long ld;
+  int ax, side;
+  double mid;
+  __device__ __forceinline__ double llo(int d) const {
+    return d == ax && side ? mid : r->lo[d];
+  }
+  __device__ __forceinline__ double lhi(int d) const {
+    return d == ax && !side ? mid : r->hi[d];
+  }
+  __device__ __forceinline__ double lo(int d) const { return fma(llo(d), bw[d * ld], bl[d * ld]); }
+  __device__ __forceinline__ double len(int d) const { return (lhi(d) - llo(d)) * bw[d * ld]; }
+  __device__ __forceinline__ int widest() const {  // GPUQuadSample.cu:118-125
+    int w = 0;
+    double m = 0;
+    for (int d = 0; d < N; ++d) {
+      const double v = lhi(d) - llo(d);
+      if (v > m) {
+        m = v;
+        w = d;
+      }
+    }
+    return w;
+  }
+};
+
+}  // namespace detail
+
+// Threads of a block of k_phase2_split, and its lanes per child (the axes
+// are dealt to them).  Few lanes per box give throughput, many a short chain
+// of dependent bisections: up to kSplitWideBoxes boxes (one integral's
+// leftovers, whose longest box sets the end) take the wide form, more the
+// narrow one.  Measured on a B200, 8 against 4 lanes: 30 k boxes of a 5-D
+// product peak 1.11 against 1.45 ms, 2.0 M boxes of 6-D ones 62.6 against
+// 55.3 ms.
+constexpr int kSplitThreads = 128;
+template <int N, bool kWide>
+constexpr int kSplitLanes = N <= 2 ? 2 : (N <= 4 || !kWide) ? 4 : 8;
+constexpr long long kSplitWideBoxes = 1 << 16;
+template <int K>
+constexpr int kSplitSmem = kSplitThreads / (2 * K) * detail::SplitHeap::kBytes;
+__host__ __device__ inline int split_stride(int max_regions) { return (max_regions + 4) & ~1; }
+
+// Depth-first refinement with 2K lanes per box: the lower K lanes evaluate
+// the lower child of each bisection, the upper K the upper one
+// (axis_split_sums), and the first lane keeps the box's heap.  A box that is
+// done gives its lanes to the next box of the work counter.
+//
+// Against a warp per box with 16 lanes per child (k_phase2), 2.0 M boxes of
+// 6-D product peaks (60 M subregions) went from 299 to 55 ms on a B200.
+// Bound by the latency of a bisection (10 k cycles when few boxes are left:
+// 3.6 k for the children's sums, 1.7 k for their errors, the rest the heap
+// and the pool) and, with all lanes busy, by the pools' traffic through L2.
+template <int N, int K, class Src>
+__global__ void __launch_bounds__(kSplitThreads, 4) k_phase2_split(Src src, RuleTables T,
+                                                                   Phase2Args a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kGroup = 2 * K;
+  __shared__ RuleTables tables;
+  detail::stage_tables(T, tables);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, gl = lane % kGroup, lead = lane - gl;
+  const int side = gl / K, j = gl % K;
+  const unsigned cmask = ((1u << K) - 1u) << (lead + side * K);  // this child's lanes
+  const bool leader = gl == 0;
+  const long long group = ((long long)blockIdx.x * kSplitThreads + threadIdx.x) / kGroup;
+  const int stride = split_stride(a.max_regions);
+  P2Region<N>* pool = reinterpret_cast<P2Region<N>*>(a.slab) + group * stride;
+  extern __shared__ __align__(16) unsigned char split_dyn[];  // SplitHeap::kBytes a group
+  detail::SplitHeap heap;
+  heap.key = reinterpret_cast<unsigned long long*>(
+      split_dyn + (threadIdx.x / kGroup) * detail::SplitHeap::kBytes);
+  heap.id = reinterpret_cast<int*>(heap.key + detail::SplitHeap::kTop);
+  heap.g = a.heap + group * stride;
+  bool more = true, have = false;
+  int box = 0, k = 0, nreg = 0, used = 0, hn = 0;
+  double epsrel = 0, epsabs = 0, ERR = 0, RESULT = 0;
+  for (;;) {
+    // a new box for every group without one
+    const bool want = more && !have;
+    const unsigned wm = __ballot_sync(kAll, want && leader);
+    if (wm) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(a.next_box, __popc(wm));
+      base = __shfl_sync(kAll, base, 0);
+      if (want) {
+        box = base + __popc(wm & ((1u << lead) - 1u));
+        have = more = box < a.n_left;
+        if (have) {
+          if (a.pair_half) box = box < a.pair_half ? 2 * box : 2 * (box - a.pair_half) + 1;
+          k = a.left_rid[box];
+          epsrel = a.ist[k].epsrel;
+          epsabs = a.ist[k].epsabs;
+          nreg = used = hn = 0;
+          // the whole box as the first subregion (INIT_REGION_POOL, :110-182)
+          for (int d = gl; d < N; d += kGroup) {
+            pool->lo[d] = 0;
+            pool->hi[d] = 1;
+          }
+        }
+      }
+    }
+    if (!__any_sync(kAll, have)) break;
+    int pi = 0;
+    if (have && nreg > 0 && leader) pi = heap.pop(hn);
+    pi = __shfl_sync(kAll, pi, lead);
+    __syncwarp();
+    const bool split = have && nreg > 0;
+    P2Region<N>* par = pool + pi;
+    int ax = -1;
+    double mid = 0, pavg = 0, perr = 0;
+    detail::RegionResult r;
+    r.avg = r.err = 0;
+    r.axis = 0;
+    if (have) {
+      if (split) {
+        ax = par->axis;
+        pavg = par->avg;
+        perr = par->err;
+        mid = 0.5 * (par->lo[ax] + par->hi[ax]);
+      }
+      const detail::SubBox<N> sb{par, a.left_lo + box, a.left_len + box, a.left_cap,
+                                 ax,  side,            mid};
+      const auto& f = detail::source_view(src, k);
+      detail::RegionSums rs;
+      double jac;
+      detail::axis_split_sums<N, K, detail::SourceFn<Src>>(f, sb, j, cmask, tables.ratio, rs, jac);
+      int fallback = 0;
+      if (rs.axis < 0) fallback = sb.widest();
+      r = detail::finish_region_split<K>(rs, tables, jac, fallback, j, cmask);
+    }
+    __syncwarp();
+    const double oavg = __shfl_xor_sync(kAll, r.avg, K);
+    const double oerr = __shfl_xor_sync(kAll, r.err, K);
+    const double avgL = side ? oavg : r.avg, avgR = side ? r.avg : oavg;
+    double errL = side ? oerr : r.err, errR = side ? r.err : oerr;
+    if (split) {
+      // Cuhre error refinement (GPUQuadPhases.cu:498-515)
+      const double diff = fabs(.25 * (avgL + avgR - pavg));
+      const double e = errL + errR;
+      if (e > 0) {
+        const double c = 1 + 2 * diff / e;
+        errL *= c;
+        errR *= c;
+      }
+      errL += diff;
+      errR += diff;
+      ERR += errL + errR - perr;
+      RESULT += avgL + avgR - pavg;
+      if (side) {
+        P2Region<N>* up = pool + used;
+        for (int d = j; d < N; d += K) {
+          up->lo[d] = d == ax ? mid : par->lo[d];
+          up->hi[d] = par->hi[d];
+        }
+        if (j == 0) {
+          up->avg = avgR;
+          up->err = errR;
+          up->axis = r.axis;
+        }
+      }
+    } else if (have) {
+      // both children's lanes evaluated the whole box
+      ERR = r.err;
+      RESULT = r.avg;
+    }
+    __syncwarp();  // the upper child has read its parent's box
+    if (have && leader) {
+      par->avg = avgL;
+      par->err = errL;
+      par->axis = r.axis;
+      if (split) par->hi[ax] = mid;
+      heap.push(hn, pi, errL);
+      if (split) heap.push(hn, used, errR);
+    }
+    if (have) {
+      ++used;
+      ++nreg;
+    }
+    if (have && !(nreg <= a.max_regions &&
+                  (nreg == 1 || ERR > detail::max_err(RESULT, epsrel, epsabs)))) {
+      have = false;
+      if (leader) {
+        int failed = ERR > detail::max_err(RESULT, epsrel, epsabs);
+        if (ERR > 1e10) {  // GPUQuadPhases.cu:519-527
+          RESULT = 0.0;
+          ERR = 0.0;
+          failed = 1;
+        }
+        LeftoverResult o;
+        o.value = RESULT;
+        o.error = ERR;
+        o.nregions = nreg;
+        o.failed = failed;
+        a.out[box] = o;
+      }
     }
     __syncwarp();
   }

@@ -239,6 +239,38 @@ struct AxisPoly {
     z *= c;
   }
 
+  // Those of two disjoint groups of axes together.
+  __device__ __forceinline__ static AxisPoly join(const AxisPoly& a, const AxisPoly& b) {
+    AxisPoly r;
+    r.e3 = fma(a.e3, b.z, fma(a.e2, b.e1, fma(a.e1, b.e2, a.z * b.e3)));
+    r.e2 = fma(a.e2, b.z, fma(a.e1, b.e1, a.z * b.e2));
+    r.g = fma(a.g, b.z, fma(a.e1, b.h1, fma(a.h1, b.e1, a.z * b.g)));
+    r.e1 = fma(a.e1, b.z, a.z * b.e1);
+    r.h1 = fma(a.h1, b.z, a.z * b.h1);
+    r.p = fma(a.p, b.z, a.z * b.p);
+    r.q = fma(a.q, b.z, a.z * b.q);
+    r.l = a.l * b.l;
+    r.z = a.z * b.z;
+    return r;
+  }
+
+  // This and the polynomials of the lane `off` above in the K-lane group
+  // (complete in lane 0 after off = 1, 2, ..., K / 2).
+  template <int K>
+  __device__ __forceinline__ void join_down(unsigned mask, int off) {
+    AxisPoly o;
+    o.z = __shfl_down_sync(mask, z, off, K);
+    o.e1 = __shfl_down_sync(mask, e1, off, K);
+    o.e2 = __shfl_down_sync(mask, e2, off, K);
+    o.e3 = __shfl_down_sync(mask, e3, off, K);
+    o.h1 = __shfl_down_sync(mask, h1, off, K);
+    o.g = __shfl_down_sync(mask, g, off, K);
+    o.p = __shfl_down_sync(mask, p, off, K);
+    o.q = __shfl_down_sync(mask, q, off, K);
+    o.l = __shfl_down_sync(mask, l, off, K);
+    *this = join(*this, o);
+  }
+
   __device__ __forceinline__ void store(RegionSums& out) const {
     out.S[0] = z;
     out.S[1] = e1;
@@ -278,6 +310,19 @@ struct AxisChoice {
       axis = d;
     } else {
       second = v <= second ? second : v;  // NaN stays
+    }
+  }
+
+  template <int K>
+  __device__ __forceinline__ void join_lanes(unsigned mask, int off) {
+    const double ob = __shfl_xor_sync(mask, best, off, K), os = __shfl_xor_sync(mask, second, off, K);
+    const int oa = __shfl_xor_sync(mask, axis, off, K);
+    scale = fmax(scale, __shfl_xor_sync(mask, scale, off, K));
+    const double m = second <= os ? os : second, lo = ob <= best ? ob : best;
+    second = m <= lo ? lo : m;
+    if (ob > best) {
+      best = ob;
+      axis = oa;
     }
   }
 
@@ -380,6 +425,33 @@ __device__ __forceinline__ void axis_product_sums(const V& f, const Box& box, do
   out.axis = ch.sure(F::kNoise, poly.z) ? ch.axis : exact_axis<N, F>(f, box, ratio);
 }
 
+// axis_product_sums with the axes dealt to the K lanes of a group (lane j:
+// axes j, j + K, ...), for chains of dependent regions, where the latency of
+// one region counts: a lane evaluates its axes' factors, and the lanes'
+// polynomials are joined by shuffles.  Every lane of the group (mask, K
+// aligned lanes) gets the sums.
+template <int N, int K, class F, class V, class Box>
+__device__ __forceinline__ void axis_split_sums(const V& f, const Box& box, int j, unsigned mask,
+                                                double ratio, RegionSums& out, double& jac) {
+  AxisPoly poly;
+  AxisChoice ch;
+  jac = 1;
+#pragma unroll 1
+  for (int d = j; d < N; d += K) append_axis<F>(f, box, d, ratio, poly, ch, jac);
+  __syncwarp(mask);
+#pragma unroll
+  for (int off = 1; off < K; off <<= 1) {
+    poly.template join_down<K>(mask, off);
+    ch.template join_lanes<K>(mask, off);
+    jac = __dmul_rn(jac, __shfl_xor_sync(mask, jac, off));
+  }
+  poly.store(out);
+#pragma unroll
+  for (int k = 0; k < kNumSets; ++k) out.S[k] = __shfl_sync(mask, out.S[k], 0, K);
+  out.best = ch.best;
+  out.axis = ch.sure(F::kNoise, out.S[0]) ? ch.axis : exact_axis<N, F>(f, box, ratio);
+}
+
 // A box in an SoA region list.
 struct ListBox {
   const double* lo0;
@@ -474,6 +546,53 @@ __device__ __forceinline__ RegionResult finish_region(const RegionSums& r, const
       m = (m > e) ? m : e;
     }
     nul[q] = m;
+  }
+  RegionResult out;
+  out.avg = sum[0];
+  const double m12 = nul[1] > nul[2] ? nul[1] : nul[2];
+  const double m123 = m12 > nul[3] ? m12 : nul[3];
+  out.err = (__dmul_rn(5.0, nul[1]) <= nul[2] && __dmul_rn(5.0, nul[2]) <= nul[3])
+                ? nul[1]
+                : __dmul_rn(5.0, m123);
+  out.axis = r.axis >= 0 ? r.axis : fallback_axis;
+  return out;
+}
+
+// finish_region with the rules dealt to the K lanes of a group, each with
+// finish_region's arithmetic for its rule.  T is read by lane index, so it
+// must lie in shared memory.  Every lane gets the result.
+template <int K>
+__device__ __forceinline__ RegionResult finish_region_split(const RegionSums& r,
+                                                            const RuleTables& T, double jac,
+                                                            int fallback_axis, int j,
+                                                            unsigned mask) {
+  double sum[kNumRules];
+#pragma unroll
+  for (int a = 0; a < (kNumRules + K - 1) / K; ++a) {
+    const int q = j + a * K < kNumRules ? j + a * K : 0;
+    double acc = 0;
+#pragma unroll
+    for (int k = 0; k < kNumSets; ++k) acc = __dadd_rn(acc, __dmul_rn(T.wt[k][q], r.S[k]));
+    acc = __dmul_rn(acc, jac);
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (a * K + i < kNumRules) sum[a * K + i] = __shfl_sync(mask, acc, i, K);
+  }
+  double nul[kNumRules];
+#pragma unroll
+  for (int a = 0; a < (kNumRules - 2 + K - 1) / K; ++a) {
+    const int q = 1 + (j + a * K < kNumRules - 2 ? j + a * K : 0);
+    const double sq = q == 1 ? sum[1] : q == 2 ? sum[2] : sum[3];
+    const double sq1 = q == 1 ? sum[2] : q == 2 ? sum[3] : sum[4];
+    double m = 0;
+#pragma unroll
+    for (int k = 0; k < kNumSets; ++k) {
+      const double e = __dmul_rn(fabs(__dadd_rn(sq1, __dmul_rn(T.scale[k][q], sq))), T.norm[k][q]);
+      m = (m > e) ? m : e;
+    }
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (a * K + i < kNumRules - 2) nul[1 + a * K + i] = __shfl_sync(mask, m, i, K);
   }
   RegionResult out;
   out.avg = sum[0];

@@ -91,6 +91,60 @@ def test_tiles_of_long_lists(cub, oracle, ctx):
         assert r.status == 0 and abs(r.integral - exact) <= max(r.error, 1e-13 * exact)
 
 
+@pytest.mark.parametrize("n", range(2, 9))
+@pytest.mark.parametrize("family", ["gaussian", "product_peak"])
+def test_second_phase_of_products(cub, oracle, ctx, family, n):
+    """The second phase with a few lanes per box, in every dimension, against
+    the oracle's (the bounds of tests/test_gpu_parity.py: values within 2
+    epsrel, region counts within 0.5%)."""
+    rng = np.random.default_rng(31 * n)
+    eps = {2: 1e-9, 3: 1e-8, 4: 1e-7, 5: 1e-6, 6: 1e-5, 7: 1e-3, 8: 1e-3}[n]
+    a = rng.uniform(8, 14, n) if family == "product_peak" else rng.uniform(6, 9, n)
+    u = rng.uniform(0.3, 0.7, n)
+    kw = dict(phase1_cap=256)
+    ctx.reset_stats()
+    r = ctx.integrate(cub.Integrand(family, n, list(a), list(u)), eps, 1e-14,
+                      cub.options(**kw))
+    assert ctx.stats()["phase2_boxes"] > 0
+    o = oracle.Rule(n).integrate_reference(oracle.make_integrand(family, n, a, u), eps, 1e-14, **kw)
+    assert r.status == o["status"]
+    assert abs(r.integral - o["value"]) <= 2 * eps * abs(o["value"])
+    assert abs(r.nregions - o["nregions"]) <= 0.005 * o["nregions"]
+
+
+@pytest.mark.parametrize("cap", [7, 254, 255, 256, 600])
+def test_second_phase_heap_sizes(cub, oracle, ctx, cap):
+    """Bisection limits around the number of heap entries kept in shared
+    memory, on boxes that reach them."""
+    n, eps = 5, 1e-8
+    a, u = [20.0, 30.0, 10.0, 25.0, 15.0], [0.3, 0.5, 0.7, 0.45, 0.6]
+    r = ctx.integrate(cub.Integrand("product_peak", n, a, u), eps, 1e-14,
+                      cub.options(phase1_cap=64, phase2_max_regions=cap))
+    o = oracle.Rule(n).integrate_reference(oracle.make_integrand("product_peak", n, a, u), eps,
+                                           1e-14, phase1_cap=64, phase2_max=cap)
+    assert r.status == o["status"] > 0
+    assert r.nregions == o["nregions"]
+    assert abs(r.integral - o["value"]) <= 1e-9 * abs(o["value"])
+
+
+def test_second_phase_wide_and_narrow(cub, ctx):
+    """Few leftover boxes take more lanes per box than many: an integral by
+    itself and in a batch whose boxes pass the limit gets the same answer."""
+    n, eps = 3, 1e-10
+    rng = np.random.default_rng(3)
+    params = [cub.make_params(n, list(rng.uniform(15, 30, n)), list(rng.uniform(0.3, 0.7, n)))
+              for _ in range(24)]
+    opts = cub.options(phase1_cap=4096)
+    ctx.reset_stats()
+    batch = ctx.integrate_batch("product_peak", n, params, eps, 1e-15, opts)
+    assert ctx.stats()["phase2_boxes"] > 1 << 16
+    for k in (0, 11, 23):
+        one = ctx.integrate_batch("product_peak", n, [params[k]], eps, 1e-15, opts)[0]
+        assert one.status == batch[k].status
+        assert abs(one.integral - batch[k].integral) <= 1e-11 * abs(one.integral)
+        assert abs(one.nregions - batch[k].nregions) <= 0.005 * one.nregions
+
+
 def test_table_regions_match_the_points(cub, oracle, ctx):
     """The table integrand by one thread per region (long lists) against the
     16- and 32-lane point-by-point forms: the same run, the same counts."""
