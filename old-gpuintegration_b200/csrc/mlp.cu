@@ -3,10 +3,12 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "capi_internal.h"
@@ -31,20 +33,34 @@ int* error_flag() {
   return flags[dev];
 }
 
-template <int N, int EPI>
-cudaError_t launch_gemm(dim3 grid, cudaStream_t s, const umma::GemmArgs& g,
-                        const mlp::EpiArgs& ep) {
-  static bool configured[64] = {};
+// Allow `kernel` its dynamic shared memory, once per device.
+template <class K>
+cudaError_t allow_smem(K kernel, int bytes, std::atomic<bool> (&done)[64]) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (!configured[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(mlp::k_gemm<N, EPI>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         mlp::kGemmSmem);
-    if (e != cudaSuccess) return e;
-    configured[dev & 63] = true;
-  }
-  mlp::k_gemm<N, EPI><<<grid, 128, mlp::kGemmSmem, s>>>(g, ep);
+  if (done[dev & 63].load(std::memory_order_relaxed)) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done[dev & 63].store(true, std::memory_order_relaxed);
+  return e;
+}
+
+template <int N>
+cudaError_t launch_gemm(dim3 grid, cudaStream_t s, const umma::GemmArgs& g, float* out,
+                        long long ld_out, long long batch_out) {
+  static std::atomic<bool> configured[64];
+  const cudaError_t e = allow_smem(mlp::k_gemm<N>, mlp::kGemmSmem, configured);
+  if (e != cudaSuccess) return e;
+  mlp::k_gemm<N><<<grid, 128, mlp::kGemmSmem, s>>>(g, out, ld_out, batch_out);
+  return cudaGetLastError();
+}
+
+template <bool kTrain>
+cudaError_t launch_net(dim3 grid, cudaStream_t s, const mlp::NetArgs& a) {
+  static std::atomic<bool> configured[64];
+  const cudaError_t e = allow_smem(mlp::k_net<kTrain>, mlp::kNetSmem<kTrain>, configured);
+  if (e != cudaSuccess) return e;
+  mlp::k_net<kTrain><<<grid, 128, mlp::kNetSmem<kTrain>, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -70,16 +86,12 @@ int cub_mlp_gemm_bf16(int batch, int m, int n, int k, const void* d_a, long long
   g.m = m;
   g.k = k;
   g.error = err;
-  mlp::EpiArgs ep{};
-  ep.out = d_d;
-  ep.ld_out = ldd;
-  ep.batch_out = ldd * m;
   const dim3 grid(m / umma::kTileM, 1, batch);
   cudaError_t e;
   if (n == 16) {
-    e = launch_gemm<16, mlp::kEpiStore>(grid, s, g, ep);
+    e = launch_gemm<16>(grid, s, g, d_d, ldd, ldd * m);
   } else {
-    e = launch_gemm<128, mlp::kEpiStore>(grid, s, g, ep);
+    e = launch_gemm<128>(grid, s, g, d_d, ldd, ldd * m);
   }
   if (e != cudaSuccess) return cuda_error(e, "k_gemm launch");
   int h_err = 0;
@@ -106,24 +118,15 @@ struct cub_mlp {
   int* err = nullptr;
   int step = 0;
   bool have_data = false;
-  std::vector<void*> bufs;
+  void* mem = nullptr;  // the one allocation all buffers are cut from
   float *P, *G, *Mm, *Vv, *part, *loss, *scale, *Y;
-  bf16 *W0, *W1, *W1T, *W2, *W2T, *X, *XT, *XE, *XET;
-  bf16 *Z1, *H1, *H1T, *Z2, *H2, *H2T, *Z3, *H3, *H3T;
-  bf16 *dZ1, *dZ1T, *dZ2, *dZ2T, *dZ3, *dZ3T;
+  bf16 *W0, *W1, *W1T, *W2, *W2T, *X, *XT;
+  bf16 *Z1, *Z2, *H1T, *H2T, *dZ1T, *dZ2T, *dZ3T;
 
-  template <class T>
-  bool alloc(T** p, size_t n) {
-    void* q = nullptr;
-    if (cudaMalloc(&q, n * sizeof(T)) != cudaSuccess) return false;
-    bufs.push_back(q);
-    *p = static_cast<T*>(q);
-    return true;
-  }
   ~cub_mlp() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    for (void* q : bufs) cudaFree(q);
+    if (mem) cudaFree(mem);
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -152,109 +155,66 @@ void init_params(std::vector<float>& p, int E, unsigned long long seed) {
 
 int check(cudaError_t e, const char* what) { return e == cudaSuccess ? 0 : cuda_error(e, what); }
 
+mlp::BfWeights bf_weights(const cub_mlp* m) { return {m->W0, m->W1, m->W1T, m->W2, m->W2T}; }
+
 int refresh(cub_mlp* m) {
-  mlp::k_refresh_weights<<<dim3(64, 1, m->E), 256, 0, m->stream>>>(m->P, m->W0, m->W1, m->W1T,
-                                                                     m->W2, m->W2T);
+  mlp::k_refresh_weights<<<592, 256, 0, m->stream>>>(m->P, (long long)m->E * Layout::kCount,
+                                                     bf_weights(m));
   return check(cudaGetLastError(), "k_refresh_weights");
 }
 
-// Forward pass of `rows` rows (multiple of 128) starting at X (row-major,
-// per-network stride batch_x): Z/H/HT of the three hidden layers.
-int forward(cub_mlp* m, const bf16* X, long long batch_x, int rows) {
-  const long long B = rows;
-  const dim3 grid(rows / umma::kTileM, 1, m->E);
-  umma::GemmArgs g{};
-  g.error = m->err;
-  g.m = rows;
-  mlp::EpiArgs ep{};
-  ep.batch_bias = Layout::kCount;
-  ep.ld_act = 128;
-  ep.batch_act = B * 128;
-  ep.ld_t = B;
-  ep.batch_t = 128 * B;
-  const bf16* in[3] = {X, m->H1, m->H2};
-  const bf16* w[3] = {m->W0, m->W1, m->W2};
-  bf16* z[3] = {m->Z1, m->Z2, m->Z3};
-  bf16* h[3] = {m->H1, m->H2, m->H3};
-  bf16* ht[3] = {m->H1T, m->H2T, m->H3T};
-  const int boff[3] = {Layout::B0, Layout::B1, Layout::B2};
-  for (int l = 0; l < 3; ++l) {
-    g.a = in[l];
-    g.lda = l == 0 ? mlp::kInPad : 128;
-    g.batch_a = l == 0 ? batch_x : B * 128;
-    g.b = w[l];
-    g.ldb = l == 0 ? mlp::kInPad : 128;
-    g.batch_b = l == 0 ? 128 * mlp::kInPad : 128 * 128;
-    g.k = l == 0 ? mlp::kInPad : 128;
-    ep.bias = m->P + boff[l];
-    ep.z = z[l];
-    ep.h = h[l];
-    ep.ht = ht[l];
-    cudaError_t e = launch_gemm<128, mlp::kEpiForward>(grid, m->stream, g, ep);
-    if (e != cudaSuccess) return cuda_error(e, "forward GEMM");
-  }
-  return 0;
+mlp::NetArgs net_args(const cub_mlp* m) {
+  mlp::NetArgs a{};
+  a.P = m->P;
+  a.W0 = m->W0;
+  a.W1 = m->W1;
+  a.W2 = m->W2;
+  a.W1T = m->W1T;
+  a.W2T = m->W2T;
+  a.error = m->err;
+  return a;
 }
 
 // Forward + backward of minibatch b into G (no update); loss into m->loss.
 int grad_step(cub_mlp* m, int b) {
-  const long long B = m->B, S = m->S;
-  const long long s0 = (long long)b * B;
-  int rc = forward(m, m->X + s0 * mlp::kInPad, S * mlp::kInPad, m->B);
+  const long long B = m->B, S = m->S, s0 = (long long)b * B;
+  const int ntiles = m->B / 128;
+  mlp::NetArgs a = net_args(m);
+  a.X = m->X + s0 * mlp::kInPad;
+  a.batch_X = S * mlp::kInPad;
+  a.y = m->Y + s0;
+  a.batch_y = S;
+  a.inv_nbatch = 1.0f / (float)m->B;
+  a.Z1 = m->Z1;
+  a.Z2 = m->Z2;
+  a.H1T = m->H1T;
+  a.H2T = m->H2T;
+  a.dZ1T = m->dZ1T;
+  a.dZ2T = m->dZ2T;
+  a.dZ3T = m->dZ3T;
+  a.part = m->part;
+  a.rows = B;
+  int rc = check(launch_net<true>(dim3(ntiles, 1, m->E), m->stream, a), "k_net");
   if (rc) return rc;
-  const int nblk = m->B / 128;
-  const float inv = 1.0f / (float)m->B;
-  mlp::k_output<<<dim3(nblk, 1, m->E), 128, 0, m->stream>>>(
-      m->P, m->H3, m->Z3, m->Y + s0, S, inv, m->dZ3, m->dZ3T, m->part, B, B, m->scale, nullptr, 0);
-  if ((rc = check(cudaGetLastError(), "k_output"))) return rc;
-  mlp::k_reduce_output<<<dim3(1, 1, m->E), 160, 0, m->stream>>>(m->part, nblk, m->G, m->loss, inv);
-  if ((rc = check(cudaGetLastError(), "k_reduce_output"))) return rc;
-  umma::GemmArgs g{};
+  mlp::GradArgs g{};
+  g.dZT[0] = m->dZ1T;
+  g.dZT[1] = m->dZ2T;
+  g.dZT[2] = m->dZ3T;
+  g.HT[0] = m->XT + s0;
+  g.HT[1] = m->H1T;
+  g.HT[2] = m->H2T;
+  g.ldx = S;
+  g.rows = B;
+  g.G = m->G;
   g.error = m->err;
-  mlp::EpiArgs ep{};
-  ep.ld_act = 128;
-  ep.batch_act = B * 128;
-  ep.ld_t = B;
-  ep.batch_t = 128 * B;
-  const bf16* dzT[3] = {m->dZ1T, m->dZ2T, m->dZ3T};
-  const bf16* hT[3] = {m->XT + s0, m->H1T, m->H2T};
-  const int woff[3] = {Layout::W0, Layout::W1, Layout::W2};
-  for (int l = 2; l >= 0; --l) {
-    // weight gradient dW_l = dZ_{l+1}^T H_l
-    g.a = dzT[l];
-    g.lda = B;
-    g.batch_a = 128 * B;
-    g.b = hT[l];
-    g.ldb = l == 0 ? S : B;
-    g.batch_b = l == 0 ? mlp::kInPad * S : 128 * B;
-    g.m = 128;
-    g.k = m->B;
-    ep.out = m->G + woff[l];
-    ep.ld_out = l == 0 ? mlp::kInPad : 128;
-    ep.batch_out = Layout::kCount;
-    cudaError_t e = l == 0 ? launch_gemm<16, mlp::kEpiStore>(dim3(1, 1, m->E), m->stream, g, ep)
-                           : launch_gemm<128, mlp::kEpiStore>(dim3(1, 1, m->E), m->stream, g, ep);
-    if (e != cudaSuccess) return cuda_error(e, "weight-gradient GEMM");
-    mlp::k_bias_grad<<<dim3(16, 1, m->E), 256, 0, m->stream>>>(dzT[l], B, m->G,
-                                                                 woff[l] + (l == 0 ? 128 * 16 : 128 * 128));
-    if ((rc = check(cudaGetLastError(), "k_bias_grad"))) return rc;
-    if (l == 0) break;
-    // dZ_l = (dZ_{l+1} W_l) * silu'(Z_l)
-    g.a = l == 2 ? m->dZ3 : m->dZ2;
-    g.lda = 128;
-    g.batch_a = B * 128;
-    g.b = l == 2 ? m->W2T : m->W1T;
-    g.ldb = 128;
-    g.batch_b = 128 * 128;
-    g.m = m->B;
-    g.k = 128;
-    ep.zin = l == 2 ? m->Z2 : m->Z1;
-    ep.dz = l == 2 ? m->dZ2 : m->dZ1;
-    ep.dzt = l == 2 ? m->dZ2T : m->dZ1T;
-    e = launch_gemm<128, mlp::kEpiBackward>(dim3(m->B / 128, 1, m->E), m->stream, g, ep);
-    if (e != cudaSuccess) return cuda_error(e, "backward GEMM");
-  }
-  return 0;
+  static std::atomic<bool> configured[64];
+  rc = check(allow_smem(mlp::k_weight_grads, mlp::kGradSmem, configured), "k_weight_grads");
+  if (rc) return rc;
+  mlp::k_weight_grads<<<dim3(3, 1, m->E), 128, mlp::kGradSmem, m->stream>>>(g);
+  if ((rc = check(cudaGetLastError(), "k_weight_grads"))) return rc;
+  mlp::k_small_grads<<<dim3(49, 1, m->E), 256, 0, m->stream>>>(g, m->part, ntiles, m->loss,
+                                                               a.inv_nbatch);
+  return check(cudaGetLastError(), "k_small_grads");
 }
 
 int read_error(cub_mlp* m) {
@@ -287,19 +247,34 @@ cub_mlp* cub_mlp_create(int device, int count, int samples, int batch, unsigned 
   m->S = samples;
   m->B = batch;
   const size_t E = count, S = samples, B = batch, P = Layout::kCount;
+  // one allocation, cut into 256-byte aligned buffers (a create and destroy
+  // of 38 allocations cost milliseconds); a first pass adds the sizes up
+  char* base = nullptr;
+  size_t used = 0;
+  auto cut = [&](auto** p, size_t n) {
+    *p = reinterpret_cast<std::remove_pointer_t<decltype(p)>>(base + used);
+    used += (n * sizeof(**p) + 255) & ~size_t(255);
+  };
+  auto layout = [&] {
+    used = 0;
+    cut(&m->err, 1);
+    for (float** q : {&m->P, &m->G, &m->Mm, &m->Vv}) cut(q, E * P);
+    cut(&m->part, E * (B / 128) * (128 + 2));
+    cut(&m->loss, E);
+    cut(&m->scale, E);
+    cut(&m->Y, E * S);
+    cut(&m->W0, E * 128 * 16);
+    for (bf16** q : {&m->W1, &m->W1T, &m->W2, &m->W2T}) cut(q, E * 128 * 128);
+    cut(&m->X, E * S * 16);
+    cut(&m->XT, E * S * 16);
+    for (bf16** q : {&m->Z1, &m->Z2, &m->H1T, &m->H2T, &m->dZ1T, &m->dZ2T, &m->dZ3T})
+      cut(q, E * B * 128);
+  };
+  layout();
   bool ok = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) == cudaSuccess &&
-            m->alloc(&m->err, 1) && m->alloc(&m->P, E * P) && m->alloc(&m->G, E * P) &&
-            m->alloc(&m->Mm, E * P) && m->alloc(&m->Vv, E * P) &&
-            m->alloc(&m->part, E * (B / 128) * (128 + 2)) && m->alloc(&m->loss, E) &&
-            m->alloc(&m->scale, E) && m->alloc(&m->Y, E * S) &&
-            m->alloc(&m->W0, E * 128 * 16) && m->alloc(&m->W1, E * 128 * 128) &&
-            m->alloc(&m->W1T, E * 128 * 128) && m->alloc(&m->W2, E * 128 * 128) &&
-            m->alloc(&m->W2T, E * 128 * 128) && m->alloc(&m->X, E * S * 16) &&
-            m->alloc(&m->XT, E * S * 16) && m->alloc(&m->XE, E * B * 16) &&
-            m->alloc(&m->XET, E * B * 16);
-  bf16** act[] = {&m->Z1, &m->H1, &m->H1T, &m->Z2, &m->H2, &m->H2T, &m->Z3, &m->H3,
-                  &m->H3T, &m->dZ1, &m->dZ1T, &m->dZ2, &m->dZ2T, &m->dZ3, &m->dZ3T};
-  for (bf16** a : act) ok = ok && m->alloc(a, E * B * 128);
+            cudaMalloc(&m->mem, used) == cudaSuccess;
+  base = static_cast<char*>(m->mem);
+  if (ok) layout();
   if (!ok) {
     set_error("cub_mlp_create: device allocation failed");
     delete m;
@@ -389,8 +364,9 @@ int cub_mlp_train(cub_mlp* m, int epochs, float lr, float* h_loss) {
       if (rc) return rc;
       ++m->step;
       const float c1 = 1.0f - std::pow(b1, (float)m->step), c2 = 1.0f - std::pow(b2, (float)m->step);
-      mlp::k_adam<<<592, 256, 0, m->stream>>>(m->P, m->G, m->Mm, m->Vv, n, lr, b1, b2, 1e-8f, c1, c2);
-      if ((rc = check(cudaGetLastError(), "k_adam")) || (rc = refresh(m))) return rc;
+      mlp::k_adam<<<592, 256, 0, m->stream>>>(m->P, m->G, m->Mm, m->Vv, n, lr, b1, b2, 1e-8f, c1,
+                                              c2, bf_weights(m));
+      if ((rc = check(cudaGetLastError(), "k_adam"))) return rc;
     }
     int rc = read_error(m);  // once per epoch
     if (rc) return rc;
@@ -406,20 +382,18 @@ int cub_mlp_eval(cub_mlp* m, long long n, const double* d_x, double* d_g) {
     return CUB_ERR_INVALID;
   }
   cudaSetDevice(m->device);
-  const long long B = m->B;
-  for (long long c0 = 0; c0 < n; c0 += B) {
-    const long long cnt = std::min(B, n - c0);
-    // stale rows past cnt are evaluated and discarded
-    mlp::k_prep_inputs<<<dim3(16, 1, m->E), 256, 0, m->stream>>>(
-        d_x + c0 * mlp::kIn, cnt, n * mlp::kIn, m->XE, m->XET, B, B * mlp::kInPad,
-        B * mlp::kInPad);
-    int rc = check(cudaGetLastError(), "k_prep_inputs");
-    if (rc || (rc = forward(m, m->XE, B * mlp::kInPad, m->B))) return rc;
-    mlp::k_output<<<dim3(m->B / 128, 1, m->E), 128, 0, m->stream>>>(
-        m->P, m->H3, m->Z3, nullptr, 0, 0.0f, nullptr, nullptr, nullptr, B, cnt, m->scale,
-        d_g + c0, n);
-    if ((rc = check(cudaGetLastError(), "k_output"))) return rc;
-  }
+  mlp::NetArgs a = net_args(m);
+  a.x = d_x;
+  a.n = n;
+  a.scale = m->scale;
+  a.g = d_g;
+  // two blocks fit on an SM; a block keeps its network's weights and walks
+  // over tiles
+  const long long tiles = (n + 127) / 128;
+  const long long blocks =
+      std::min<long long>(tiles, std::max(1, (2 * sm_count(m->device) + m->E - 1) / m->E));
+  const int rc = check(launch_net<false>(dim3((unsigned)blocks, 1, m->E), m->stream, a), "k_net");
+  if (rc) return rc;
   return read_error(m);
 }
 
