@@ -478,29 +478,55 @@ __global__ void __launch_bounds__(256) k_eval_cv(F f, double ca, double cb, cons
 // FP32 activations and FP32 arithmetic on the CUDA cores (the tensor-core
 // path rounds every activation to bf16, a quantisation of ~2^-8 relative
 // that no bisection resolves, so an adaptive rule cannot converge on it).
-// One warp per node; the weights sit transposed in shared memory
-// (W^T[in][out]: lanes read consecutive outputs).  g[r] for the nodes of
-// slots [s0, s0 + n), row (s - s0) * npts + p.
-constexpr int kSmoothSmem = (16 * 128 + 2 * 128 * 128 + 4 * 128 + 8 * 2 * 128) * 4;
+// 128 nodes per block at a time: the weights sit transposed in shared memory
+// (W^T[in][out]), the nodes' activations beside them ([unit][node]), and a
+// thread accumulates 8 nodes x 8 units in registers, so a unit step costs it
+// four 16-byte loads for 64 FMAs (a warp per node reloaded every weight for
+// every node: 24.4 M nodes took 130 ms, bound by shared memory).  Each sum
+// runs over the inputs in order, starting from the bias.  g[r] for the nodes
+// of slots [s0, s0 + n), row (s - s0) * npts + p.
+constexpr int kSmoothNodes = 128;
+constexpr int kSmoothLd = kSmoothNodes + 4;  // row of the activations (16-byte aligned)
+constexpr int kSmoothSmem =
+    (16 * 128 + 2 * 128 * 128 + 4 * 128 + 128 * kSmoothLd + 8 * kSmoothNodes) * 4;
+
+// acc[8 nodes][8 units] += W^T[i][unit] * h[i][node], i = 0 .. n-1 in order.
+__device__ __forceinline__ void smooth_layer(float (&acc)[8][8], const float* wt, const float* h,
+                                             int ld, int n) {
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) {
+    const float4 a0 = *reinterpret_cast<const float4*>(h + i * ld);
+    const float4 a1 = *reinterpret_cast<const float4*>(h + i * ld + 4);
+    const float4 b0 = *reinterpret_cast<const float4*>(wt + i * 128);
+    const float4 b1 = *reinterpret_cast<const float4*>(wt + i * 128 + 4);
+    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(b[q], a[p], acc[p][q]);
+  }
+}
 
 __global__ void __launch_bounds__(256) k_cv_smooth(const float* P, const bf16* W0, const bf16* W1,
                                                    const bf16* W2, float scale, const double* lo,
                                                    const double* len, const int* rid,
                                                    long long cap, long long s0, long long n,
                                                    double* g) {
-  extern __shared__ float fsm[];
-  float* w0t = fsm;                 // [16][128]
-  float* w1t = w0t + 16 * 128;      // [128][128]
-  float* w2t = w1t + 128 * 128;     // [128][128]
-  float* bias = w2t + 128 * 128;    // b0, b1, b2, w3
-  float* buf = bias + 4 * 128;      // per warp: two rows of 128
+  extern __shared__ __align__(16) float fsm[];
+  float* w0t = fsm;                         // [16][128]
+  float* w1t = w0t + 16 * 128;              // [128][128]
+  float* w2t = w1t + 128 * 128;             // [128][128]
+  float* bias = w2t + 128 * 128;            // b0, b1, b2, w3
+  float* act = bias + 4 * 128;              // [128 units][kSmoothLd]
+  float* xs = act + 128 * kSmoothLd;        // [8 inputs][128 nodes]
   __shared__ CvPT pt;
   pt.fill(threadIdx.x, blockDim.x);
   for (int i = threadIdx.x; i < 128 * 128; i += blockDim.x) {
-    const int o = i / 128, in = i % 128;
-    w1t[in * 128 + o] = __bfloat162float(W1[i]);
-    w2t[in * 128 + o] = __bfloat162float(W2[i]);
-    if (i < 128 * 16) w0t[(i % 16) * 128 + i / 16] = __bfloat162float(W0[i]);
+    const int o = i % 128, in = i / 128;
+    w1t[i] = __bfloat162float(W1[o * 128 + in]);
+    w2t[i] = __bfloat162float(W2[o * 128 + in]);
+    if (i < 128 * 16) w0t[i] = __bfloat162float(W0[o * 16 + in]);
   }
   for (int j = threadIdx.x; j < 128; j += blockDim.x) {
     bias[j] = P[Layout::B0 + j];
@@ -510,60 +536,75 @@ __global__ void __launch_bounds__(256) k_cv_smooth(const float* P, const bf16* W
   }
   __syncthreads();
   const float b3 = P[Layout::B3];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* ha = buf + warp * 256;
-  float* hb = ha + 128;
+  const int u0 = (threadIdx.x & 15) * 8, n0 = (threadIdx.x >> 4) * 8;  // this thread's tile
   const long long nodes = n * CvPT::kPoints;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long r = (long long)blockIdx.x * (blockDim.x >> 5) + warp; r < nodes; r += nwarps) {
-    const long long s = s0 + r / CvPT::kPoints;
-    if (rid[s] < 0) {
-      if (lane == 0) g[r] = 0.0;
-      continue;
+  for (long long base = (long long)blockIdx.x * kSmoothNodes; base < nodes;
+       base += (long long)gridDim.x * kSmoothNodes) {
+    if (threadIdx.x < kSmoothNodes) {
+      const long long r = base + threadIdx.x;
+      const long long s = s0 + r / CvPT::kPoints;
+      const bool live = r < nodes && rid[s] >= 0;
+      const uint2 e = pt.ent[(int)(r % CvPT::kPoints)];
+#pragma unroll
+      for (int i = 0; i < kCvDim; ++i) {
+        const double x = live ? fma(pt.ctab[(e.x >> (4 * i)) & 15u], len[(long long)i * cap + s],
+                                    lo[(long long)i * cap + s])
+                              : 0.0;
+        xs[i * kSmoothNodes + threadIdx.x] = (float)(2.0 * x - 1.0);
+      }
     }
-    const uint2 e = pt.ent[(int)(r % CvPT::kPoints)];
-    float xin[kCvDim];
+    __syncthreads();
+#pragma unroll 1
+    for (int l = 0; l < 3; ++l) {
+      float acc[8][8];
 #pragma unroll
-    for (int i = 0; i < kCvDim; ++i) {
-      const double x = fma(pt.ctab[(e.x >> (4 * i)) & 15u], len[(long long)i * cap + s],
-                           lo[(long long)i * cap + s]);
-      xin[i] = (float)(2.0 * x - 1.0);
+      for (int q = 0; q < 8; ++q) {
+        const float b = bias[l * 128 + u0 + q];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) acc[p][q] = b;
+      }
+      if (l == 0)
+        smooth_layer(acc, w0t + u0, xs + n0, kSmoothNodes, kCvDim);
+      else
+        smooth_layer(acc, (l == 1 ? w1t : w2t) + u0, act + n0, kSmoothLd, 128);
+      __syncthreads();  // every thread has read the layer's inputs
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+#pragma unroll
+        for (int p = 0; p < 8; ++p) acc[p][q] = mlp::silu(acc[p][q]);
+        float* d = act + (u0 + q) * kSmoothLd + n0;
+        *reinterpret_cast<float4*>(d) = make_float4(acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
+        *reinterpret_cast<float4*>(d + 4) = make_float4(acc[4][q], acc[5][q], acc[6][q], acc[7][q]);
+      }
+      __syncthreads();
     }
+    // Output layer, two threads per node: 32 interleaved partial sums of four
+    // units each, added as a tree over the partials' index bits from the top
+    // (16, 8, 4, 2) down; a thread holds those of one parity.
+    {
+      const int node = threadIdx.x >> 1, par = threadIdx.x & 1;
+      const float* h = act + node;
+      const float* w3 = bias + 384;
+      float t[16];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = lane + 32 * q;
-      float z = bias[j];
+      for (int v = 0; v < 16; ++v) {
+        const int l = 2 * v + par;
+        float a = 0;
 #pragma unroll
-      for (int i = 0; i < kCvDim; ++i) z = fmaf(w0t[i * 128 + j], xin[i], z);
-      ha[j] = mlp::silu(z);
-    }
-    __syncwarp();
-    const float* wt[2] = {w1t, w2t};
-    float* src = ha;
-    float* dst = hb;
-    for (int l = 0; l < 2; ++l) {
-      float z[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) z[q] = bias[128 * (l + 1) + lane + 32 * q];
-      for (int i = 0; i < 128; ++i) {
-        const float h = src[i];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) z[q] = fmaf(wt[l][i * 128 + lane + 32 * q], h, z[q]);
+        for (int q = 0; q < 4; ++q) a = fmaf(w3[l + 32 * q], h[(l + 32 * q) * kSmoothLd], a);
+        t[v] = a;
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) dst[lane + 32 * q] = mlp::silu(z[q]);
-      __syncwarp();
-      float* t = src;
-      src = dst;
-      dst = t;
+      for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          if (v < o) t[v] += t[v + o];
+      const float sum = t[0] + __shfl_xor_sync(0xffffffffu, t[0], 1);
+      const long long r = base + node;
+      if (par == 0 && r < nodes)
+        g[r] = rid[s0 + r / CvPT::kPoints] < 0 ? 0.0 : (double)scale * (double)(sum + b3);
     }
-    float acc = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc = fmaf(bias[384 + lane + 32 * q], src[lane + 32 * q], acc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) g[r] = (double)scale * (double)(acc + b3);
-    __syncwarp();
+    __syncthreads();  // the next tile overwrites the activations
   }
 }
 
