@@ -187,16 +187,20 @@ __device__ __forceinline__ __nv_bfloat16 unpack_bf16(uint32_t w, int hi) {
   return __ushort_as_bfloat16((unsigned short)(hi ? w >> 16 : w & 0xffffu));
 }
 
-// One 128-sample tile (128 threads, thread t owns row t of the tile).  The
+// One 128-sample tile, 512 threads: thread t owns row t % 128 of the tile and,
+// in the epilogues, 32 of its 128 columns (four warps share each quarter of
+// the accumulators' lanes; with one thread per row the five epilogues were a
+// chain of 128 sigmoids each and took 108 us of a step).  The
 // activations go from the accumulators (TMEM) through the epilogue straight
 // into the next product's A operand in shared memory, so a step is one launch
 // for what took eight (and the transposes, which the weight gradients read,
 // are the only activations written): 820 us a training step before, of which
 // the three forward products took 3 x 78 us on scattered 2-byte stores.
-// Bound now by the epilogues (128 sigmoids per thread and layer) and by the
-// serial chain of five products.
+// Bound now by the serial chain of five products and their epilogues.
+constexpr int kNetThreads = 512;
+
 template <bool kTrain>
-__global__ void __launch_bounds__(128) k_net(NetArgs g) {
+__global__ void __launch_bounds__(kNetThreads) k_net(NetArgs g) {
   extern __shared__ __align__(1024) uint8_t dsm[];
   uint8_t* act = dsm;
   uint8_t* xin = act + kActBytes;
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
   __shared__ uint32_t tmem_base;
   __shared__ float bias[3][kHidden], w3[kHidden], es[kHidden], sq[kHidden];
   const int e = blockIdx.z, t = threadIdx.x;
+  const int r = t & 127, c0 = (t >> 7) * 32;  // this thread's row and columns
   const float* p = g.P + (long long)e * Layout::kCount;
   stage_async(w0, g.W0 + (long long)e * kHidden * kInPad, 128, kInPad);
   stage_async(w1, g.W1 + (long long)e * kHidden * kHidden, 128, 128);
@@ -217,10 +222,12 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
     stage_async(w1t, g.W1T + (long long)e * kHidden * kHidden, 128, 128);
     stage_async(w2t, g.W2T + (long long)e * kHidden * kHidden, 128, 128);
   }
-  bias[0][t] = p[Layout::B0 + t];
-  bias[1][t] = p[Layout::B1 + t];
-  bias[2][t] = p[Layout::B2 + t];
-  w3[t] = p[Layout::W3 + t];
+  if (t < kHidden) {
+    bias[0][t] = p[Layout::B0 + t];
+    bias[1][t] = p[Layout::B1 + t];
+    bias[2][t] = p[Layout::B2 + t];
+    w3[t] = p[Layout::W3 + t];
+  }
   const float b3 = p[Layout::B3];
   if (t == 0) umma::mbar_init(&bar, 1);
   if (t < 32) umma::tmem_alloc(&tmem_base, 128);
@@ -228,7 +235,7 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = tmem_base;
-  const uint32_t lane_addr = tmem + ((uint32_t)((t >> 5) * 32) << 16);
+  const uint32_t lane_addr = tmem + ((uint32_t)((r >> 5) * 32) << 16);
   uint32_t phase = 0;
   bool ok = true;
   // one product and its wait; false (for the whole block) when it gave up
@@ -242,19 +249,20 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
     umma::fence_after_sync();
     return ok;
   };
-  // eight columns of this thread's row into the A operand
-  auto put8 = [&](int c, uint4 v) {
-    *reinterpret_cast<uint4*>(act + umma::chunk_offset(128, t, c)) = v;
+  // this thread's 32 columns into the A operand
+  auto put = [&](const uint32_t (&w)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<uint4*>(act + umma::chunk_offset(128, r, c0 + 8 * i)) =
+          make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
   };
   const long long tiles = kTrain ? gridDim.x : (g.n + 127) / 128;
   for (long long tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-    const long long row = tile * 128 + t;
+    const long long row = tile * 128 + r;
     if (kTrain) {
       stage_async(xin, g.X + (long long)e * g.batch_X + tile * 128 * kInPad, 128, kInPad);
-    } else {
-      uint32_t w[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) w[i] = 0;
+    } else if (t < 128) {
+      uint32_t w[4] = {0, 0, 0, 0};
       if (row < g.n) {
         const double* x = g.x + ((long long)e * g.n + row) * kIn;
         __nv_bfloat16 b[8];
@@ -264,72 +272,78 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = pack_bf16(b[2 * i], b[2 * i + 1]);
       }
-      *reinterpret_cast<uint4*>(xin + umma::chunk_offset(128, t, 0)) =
+      *reinterpret_cast<uint4*>(xin + umma::chunk_offset(128, r, 0)) =
           make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(xin + umma::chunk_offset(128, t, 8)) =
-          make_uint4(w[4], w[5], w[6], w[7]);
+      *reinterpret_cast<uint4*>(xin + umma::chunk_offset(128, r, 8)) = make_uint4(0, 0, 0, 0);
     }
     umma::cp_async_wait_all();
-    float out = b3;  // the output layer, columns in order
-    const long long zrow = ((long long)e * g.rows + row) * kHidden;
-    const long long trow = (long long)e * g.rows * kHidden + row;
+    const long long zrow = ((long long)e * g.rows + row) * kHidden + c0;
+    const long long trow = ((long long)e * kHidden + c0) * g.rows + row;
 #pragma unroll 1
     for (int l = 0; l < 3; ++l) {
       if (!product(l == 0 ? xin : act, l == 0 ? w0 : l == 1 ? w1 : w2, l == 0 ? 1 : 8)) break;
       __nv_bfloat16* Z = l == 0 ? g.Z1 : g.Z2;
       __nv_bfloat16* HT = l == 0 ? g.H1T : g.H2T;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 128; c0 += 32) {
-        float v[32];
-        umma::tmem_load32(lane_addr + c0, v);
-        uint32_t zw[16], hw[16];
+      float v[32];
+      umma::tmem_load32(lane_addr + c0, v);
+      uint32_t zw[16], hw[16];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          __nv_bfloat16 zb[2], hb[2];
+      for (int i = 0; i < 32; i += 2) {
+        __nv_bfloat16 zb[2], hb[2];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            zb[u] = __float2bfloat16(v[i + u] + bias[l][c0 + i + u]);
-            hb[u] = __float2bfloat16(silu(__bfloat162float(zb[u])));
-            if (l == 2) out += __bfloat162float(hb[u]) * w3[c0 + i + u];
-            if (kTrain && l < 2) HT[trow + (long long)(c0 + i + u) * g.rows] = hb[u];
-          }
-          zw[i / 2] = pack_bf16(zb[0], zb[1]);
-          hw[i / 2] = pack_bf16(hb[0], hb[1]);
+        for (int u = 0; u < 2; ++u) {
+          zb[u] = __float2bfloat16(v[i + u] + bias[l][c0 + i + u]);
+          hb[u] = __float2bfloat16(silu(__bfloat162float(zb[u])));
+          if (kTrain && l < 2) HT[trow + (long long)(i + u) * g.rows] = hb[u];
         }
-        if (kTrain || l < 2) {
+        zw[i / 2] = pack_bf16(zb[0], zb[1]);
+        hw[i / 2] = pack_bf16(hb[0], hb[1]);
+      }
+      put(hw);
+      if (kTrain && l < 2) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            put8(c0 + 8 * i, make_uint4(hw[4 * i], hw[4 * i + 1], hw[4 * i + 2], hw[4 * i + 3]));
-        }
-        if (kTrain && l < 2) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(Z + zrow + c0 + 8 * i) =
-                make_uint4(zw[4 * i], zw[4 * i + 1], zw[4 * i + 2], zw[4 * i + 3]);
-        }
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(Z + zrow + 8 * i) =
+              make_uint4(zw[4 * i], zw[4 * i + 1], zw[4 * i + 2], zw[4 * i + 3]);
       }
     }
     if (!ok) break;
-    if constexpr (!kTrain) {
-      if (row < g.n)
-        g.g[(long long)e * g.n + row] = (double)g.scale[e] * (double)out;
-    } else {
-      // loss and the output layer: err = g - y, e = 2 err / nbatch
-      const float err = out - g.y[(long long)e * g.batch_y + row];
-      const float ec = 2.0f * err * g.inv_nbatch;
-      es[t] = ec;
-      sq[t] = err * err;
+    __syncthreads();
+    // the output layer, a thread per row, columns in order
+    if (t < 128) {
+      float out = b3;
+#pragma unroll 4
+      for (int c = 0; c < 128; c += 8) {
+        const uint4 q = *reinterpret_cast<const uint4*>(act + umma::chunk_offset(128, r, c));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          out += __bfloat162float(unpack_bf16(w[i / 2], i & 1)) * w3[c + i];
+      }
+      if constexpr (!kTrain) {
+        if (row < g.n) g.g[(long long)e * g.n + row] = (double)g.scale[e] * (double)out;
+      } else {
+        // loss: err = g - y, e = 2 err / nbatch
+        const float err = out - g.y[(long long)e * g.batch_y + row];
+        es[t] = 2.0f * err * g.inv_nbatch;
+        sq[t] = err * err;
+      }
+    }
+    if constexpr (kTrain) {
       __syncthreads();
-      // this tile's partial sums (fixed order): sum_s e H3[s][:], sum_s e,
-      // sum_s err^2
+      // this tile's partial sums (fixed order): sum_s e H3[s][:] by the first
+      // 128 threads, sum_s e and sum_s err^2 by another warp's first thread
       float* po = g.part + ((long long)e * gridDim.x + blockIdx.x) * (kHidden + 2);
-      float acc = 0;
-      for (int i = 0; i < 128; ++i)
-        acc += es[i] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
-                           act + umma::chunk_offset(128, i, t)));
-      po[t] = acc;
-      if (t == 0) {
+      if (t < 128) {
+        float acc = 0;
+#pragma unroll 8
+        for (int i = 0; i < 128; ++i)
+          acc += es[i] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
+                             act + umma::chunk_offset(128, i, t)));
+        po[t] = acc;
+      } else if (t == 128) {
         float se = 0, ss = 0;
+#pragma unroll 8
         for (int i = 0; i < 128; ++i) {
           se += es[i];
           ss += sq[i];
@@ -337,6 +351,7 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
         po[kHidden] = se;
         po[kHidden + 1] = ss;
       }
+      const float ec = es[r];
       __syncthreads();  // H3 is read; its tile becomes dZ3
 #pragma unroll 1
       for (int l = 2; l >= 0; --l) {
@@ -345,44 +360,37 @@ __global__ void __launch_bounds__(128) k_net(NetArgs g) {
         if (l < 2 && !product(act, l == 1 ? w2t : w1t, 8)) break;
         __nv_bfloat16* T = l == 2 ? g.dZ3T : l == 1 ? g.dZ2T : g.dZ1T;
         const __nv_bfloat16* Z = l == 1 ? g.Z2 : g.Z1;
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-          float v[32];
-          umma::tmem_load32(lane_addr + c0, v);
-          uint32_t zw[16], dw[16];
-          if (l < 2) {
+        uint32_t zw[16], dw[16];
+        if (l < 2) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint4 q = *reinterpret_cast<const uint4*>(Z + zrow + c0 + 8 * i);
-              zw[4 * i] = q.x;
-              zw[4 * i + 1] = q.y;
-              zw[4 * i + 2] = q.z;
-              zw[4 * i + 3] = q.w;
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            __nv_bfloat16 db[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              float dz;
-              if (l == 2) {
-                const __nv_bfloat16 zb = __float2bfloat16(v[i + u] + bias[2][c0 + i + u]);
-                dz = ec * w3[c0 + i + u] * silu_grad(__bfloat162float(zb));
-              } else {
-                dz = v[i + u] * silu_grad(__bfloat162float(unpack_bf16(zw[i / 2], u)));
-              }
-              db[u] = __float2bfloat16(dz);
-              T[trow + (long long)(c0 + i + u) * g.rows] = db[u];
-            }
-            dw[i / 2] = pack_bf16(db[0], db[1]);
-          }
-          if (l > 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              put8(c0 + 8 * i, make_uint4(dw[4 * i], dw[4 * i + 1], dw[4 * i + 2], dw[4 * i + 3]));
+          for (int i = 0; i < 4; ++i) {
+            const uint4 q = *reinterpret_cast<const uint4*>(Z + zrow + 8 * i);
+            zw[4 * i] = q.x;
+            zw[4 * i + 1] = q.y;
+            zw[4 * i + 2] = q.z;
+            zw[4 * i + 3] = q.w;
           }
         }
+        float v[32];
+        umma::tmem_load32(lane_addr + c0, v);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          __nv_bfloat16 db[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            float dz;
+            if (l == 2) {
+              const __nv_bfloat16 zb = __float2bfloat16(v[i + u] + bias[2][c0 + i + u]);
+              dz = ec * w3[c0 + i + u] * silu_grad(__bfloat162float(zb));
+            } else {
+              dz = v[i + u] * silu_grad(__bfloat162float(unpack_bf16(zw[i / 2], u)));
+            }
+            db[u] = __float2bfloat16(dz);
+            T[trow + (long long)(i + u) * g.rows] = db[u];
+          }
+          dw[i / 2] = pack_bf16(db[0], db[1]);
+        }
+        if (l > 0) put(dw);
       }
     }
   }
@@ -573,6 +581,46 @@ __global__ void k_refresh_weights(const float* P, long long n, BfWeights w) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     w.put((int)(i / Layout::kCount), (int)(i % Layout::kCount), P[i]);
+}
+
+// Starting parameters: the draws of a 64-bit LCG (x -> kLcgA x + kLcgC from x0,
+// the uniform value in the high 53 bits), in the order of networks, then W0
+// (seven of sixteen columns), W1, W2, w3; uniform in +-1/sqrt(fan in), zero
+// biases and padding.  A thread jumps to its first draw (repeated squaring of
+// the step) and walks kInitRun of them: the host took 80 us a network for the
+// same serial sequence.
+constexpr unsigned long long kLcgA = 6364136223846793005ull, kLcgC = 1442695040888963407ull;
+constexpr int kInitDraws = kHidden * kIn + 2 * kHidden * kHidden + kHidden;  // per network
+constexpr int kInitRun = 32;
+
+__global__ void k_init_params(float* P, int count, unsigned long long x0) {
+  const long long total = (long long)count * kInitDraws;
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kInitRun;
+  if (first >= total) return;
+  // x0 after `first` steps
+  unsigned long long a = kLcgA, c = kLcgC, x = x0;
+  for (unsigned long long n = (unsigned long long)first; n; n >>= 1) {
+    if (n & 1) x = a * x + c;
+    c = (a + 1) * c;
+    a = a * a;
+  }
+  const double a0 = 1.0 / sqrt((double)kIn), ah = 1.0 / sqrt(128.0);
+  for (long long d = first; d < first + kInitRun && d < total; ++d) {
+    x = kLcgA * x + kLcgC;
+    const double u = (double)(x >> 11) * (1.0 / 9007199254740992.0);
+    int i = (int)(d % kInitDraws), at;
+    const bool in = i < kHidden * kIn;
+    if (in) {
+      at = Layout::W0 + i / kIn * kInPad + i % kIn;
+    } else if ((i -= kHidden * kIn) < kHidden * kHidden) {
+      at = Layout::W1 + i;
+    } else if ((i -= kHidden * kHidden) < kHidden * kHidden) {
+      at = Layout::W2 + i;
+    } else {
+      at = Layout::W3 + i - kHidden * kHidden;
+    }
+    P[d / kInitDraws * Layout::kCount + at] = (float)((2 * u - 1) * (in ? a0 : ah));
+  }
 }
 
 // Targets of network e scaled by 1 / max |y| (scale[e] = max |y|, 1 if 0).

@@ -60,7 +60,7 @@ cudaError_t launch_net(dim3 grid, cudaStream_t s, const mlp::NetArgs& a) {
   static std::atomic<bool> configured[64];
   const cudaError_t e = allow_smem(mlp::k_net<kTrain>, mlp::kNetSmem<kTrain>, configured);
   if (e != cudaSuccess) return e;
-  mlp::k_net<kTrain><<<grid, 128, mlp::kNetSmem<kTrain>, s>>>(a);
+  mlp::k_net<kTrain><<<grid, mlp::kNetThreads, mlp::kNetSmem<kTrain>, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -132,26 +132,6 @@ struct cub_mlp {
 };
 
 namespace {
-
-// Uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights from a 64-bit LCG on
-// the host, zero biases and zero padding columns of W0.
-void init_params(std::vector<float>& p, int E, unsigned long long seed) {
-  p.assign((size_t)E * Layout::kCount, 0.0f);
-  unsigned long long x = seed * 6364136223846793005ull + 1442695040888963407ull;
-  auto uni = [&x]() {
-    x = x * 6364136223846793005ull + 1442695040888963407ull;
-    return (double)(x >> 11) * (1.0 / 9007199254740992.0);
-  };
-  for (int e = 0; e < E; ++e) {
-    float* q = p.data() + (size_t)e * Layout::kCount;
-    const double a0 = 1.0 / std::sqrt((double)mlp::kIn), a = 1.0 / std::sqrt(128.0);
-    for (int o = 0; o < 128; ++o)
-      for (int i = 0; i < mlp::kIn; ++i) q[Layout::W0 + o * mlp::kInPad + i] = (float)((2 * uni() - 1) * a0);
-    for (int i = 0; i < 128 * 128; ++i) q[Layout::W1 + i] = (float)((2 * uni() - 1) * a);
-    for (int i = 0; i < 128 * 128; ++i) q[Layout::W2 + i] = (float)((2 * uni() - 1) * a);
-    for (int i = 0; i < 128; ++i) q[Layout::W3 + i] = (float)((2 * uni() - 1) * a);
-  }
-}
 
 int check(cudaError_t e, const char* what) { return e == cudaSuccess ? 0 : cuda_error(e, what); }
 
@@ -280,15 +260,16 @@ cub_mlp* cub_mlp_create(int device, int count, int samples, int batch, unsigned 
     delete m;
     return nullptr;
   }
-  std::vector<float> p;
-  init_params(p, count, seed);
-  ok = cudaMemsetAsync(m->err, 0, sizeof(int), m->stream) == cudaSuccess &&
-       cudaMemcpyAsync(m->P, p.data(), sizeof(float) * E * P, cudaMemcpyHostToDevice,
-                       m->stream) == cudaSuccess &&
-       cudaMemsetAsync(m->G, 0, sizeof(float) * E * P, m->stream) == cudaSuccess &&
-       cudaMemsetAsync(m->Mm, 0, sizeof(float) * E * P, m->stream) == cudaSuccess &&
-       cudaMemsetAsync(m->Vv, 0, sizeof(float) * E * P, m->stream) == cudaSuccess &&
-       refresh(m) == 0 && cudaStreamSynchronize(m->stream) == cudaSuccess;
+  const long long runs = ((long long)count * mlp::kInitDraws + mlp::kInitRun - 1) / mlp::kInitRun;
+  ok = cudaMemsetAsync(m->err, 0, sizeof(int), m->stream) == cudaSuccess;
+  for (float* q : {m->P, m->G, m->Mm, m->Vv})
+    ok = ok && cudaMemsetAsync(q, 0, sizeof(float) * E * P, m->stream) == cudaSuccess;
+  if (ok) {
+    mlp::k_init_params<<<(unsigned)((runs + 127) / 128), 128, 0, m->stream>>>(
+        m->P, count, seed * mlp::kLcgA + mlp::kLcgC);
+    ok = cudaGetLastError() == cudaSuccess && refresh(m) == 0 &&
+         cudaStreamSynchronize(m->stream) == cudaSuccess;
+  }
   if (!ok) {
     set_error("cub_mlp_create: initialisation failed");
     delete m;
@@ -490,21 +471,35 @@ constexpr int kSmoothLd = kSmoothNodes + 4;  // row of the activations (16-byte 
 constexpr int kSmoothSmem =
     (16 * 128 + 2 * 128 * 128 + 4 * 128 + 128 * kSmoothLd + 8 * kSmoothNodes) * 4;
 
-// acc[8 nodes][8 units] += W^T[i][unit] * h[i][node], i = 0 .. n-1 in order.
-__device__ __forceinline__ void smooth_layer(float (&acc)[8][8], const float* wt, const float* h,
+// Two FP32 FMAs in one instruction (each rounded as fmaf).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
+        "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return *reinterpret_cast<float2*>(&r);
+}
+
+// acc[node][unit pair] += W^T[i][unit] * h[i][node], i = 0 .. n-1 in order, for
+// nodes 0..3 and 64..67 of h and units 0..3 and 64..67 of wt (16-byte loads of
+// neighbouring threads are then contiguous).
+__device__ __forceinline__ void smooth_layer(float2 (&acc)[8][4], const float* wt, const float* h,
                                              int ld, int n) {
 #pragma unroll 4
   for (int i = 0; i < n; ++i) {
     const float4 a0 = *reinterpret_cast<const float4*>(h + i * ld);
-    const float4 a1 = *reinterpret_cast<const float4*>(h + i * ld + 4);
+    const float4 a1 = *reinterpret_cast<const float4*>(h + i * ld + 64);
     const float4 b0 = *reinterpret_cast<const float4*>(wt + i * 128);
-    const float4 b1 = *reinterpret_cast<const float4*>(wt + i * 128 + 4);
+    const float4 b1 = *reinterpret_cast<const float4*>(wt + i * 128 + 64);
     const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-    const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w),
+                         make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
 #pragma unroll
     for (int p = 0; p < 8; ++p)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(b[q], a[p], acc[p][q]);
+      for (int q = 0; q < 4; ++q) acc[p][q] = fma2(b[q], make_float2(a[p], a[p]), acc[p][q]);
   }
 }
 
@@ -536,7 +531,7 @@ __global__ void __launch_bounds__(256) k_cv_smooth(const float* P, const bf16* W
   }
   __syncthreads();
   const float b3 = P[Layout::B3];
-  const int u0 = (threadIdx.x & 15) * 8, n0 = (threadIdx.x >> 4) * 8;  // this thread's tile
+  const int u0 = (threadIdx.x & 15) * 4, n0 = (threadIdx.x >> 4) * 4;  // this thread's tile
   const long long nodes = n * CvPT::kPoints;
   for (long long base = (long long)blockIdx.x * kSmoothNodes; base < nodes;
        base += (long long)gridDim.x * kSmoothNodes) {
@@ -556,12 +551,13 @@ __global__ void __launch_bounds__(256) k_cv_smooth(const float* P, const bf16* W
     __syncthreads();
 #pragma unroll 1
     for (int l = 0; l < 3; ++l) {
-      float acc[8][8];
+      float2 acc[8][4];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float b = bias[l * 128 + u0 + q];
+      for (int q = 0; q < 4; ++q) {
+        const float* b = bias + l * 128 + u0 + (q >> 1) * 64 + (q & 1) * 2;
+        const float2 b2 = make_float2(b[0], b[1]);
 #pragma unroll
-        for (int p = 0; p < 8; ++p) acc[p][q] = b;
+        for (int p = 0; p < 8; ++p) acc[p][q] = b2;
       }
       if (l == 0)
         smooth_layer(acc, w0t + u0, xs + n0, kSmoothNodes, kCvDim);
@@ -569,12 +565,18 @@ __global__ void __launch_bounds__(256) k_cv_smooth(const float* P, const bf16* W
         smooth_layer(acc, (l == 1 ? w1t : w2t) + u0, act + n0, kSmoothLd, 128);
       __syncthreads();  // every thread has read the layer's inputs
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+      for (int q = 0; q < 4; ++q) {
+        float* d = act + (u0 + (q >> 1) * 64 + (q & 1) * 2) * kSmoothLd + n0;
 #pragma unroll
-        for (int p = 0; p < 8; ++p) acc[p][q] = mlp::silu(acc[p][q]);
-        float* d = act + (u0 + q) * kSmoothLd + n0;
-        *reinterpret_cast<float4*>(d) = make_float4(acc[0][q], acc[1][q], acc[2][q], acc[3][q]);
-        *reinterpret_cast<float4*>(d + 4) = make_float4(acc[4][q], acc[5][q], acc[6][q], acc[7][q]);
+        for (int p = 0; p < 8; ++p)
+          acc[p][q] = make_float2(mlp::silu(acc[p][q].x), mlp::silu(acc[p][q].y));
+#pragma unroll
+        for (int p = 0; p < 8; p += 4) {
+          *reinterpret_cast<float4*>(d + p * 16) =
+              make_float4(acc[p][q].x, acc[p + 1][q].x, acc[p + 2][q].x, acc[p + 3][q].x);
+          *reinterpret_cast<float4*>(d + kSmoothLd + p * 16) =
+              make_float4(acc[p][q].y, acc[p + 1][q].y, acc[p + 2][q].y, acc[p + 3][q].y);
+        }
       }
       __syncthreads();
     }
