@@ -400,18 +400,19 @@ __global__ void __launch_bounds__(128, kShared ? 2 : 3) k_phase2(Src src, RuleTa
 namespace detail {
 
 // Binary max-heap of one box, the comparisons of heap_push / heap_pop (same
-// bisection order).  The first kTop entries (eight levels, the whole heap of
-// most boxes) lie in shared memory, the others in global memory: entry i at
+// bisection order).  The first kTop entries (seven or eight levels, the whole
+// heap of most boxes) lie in shared memory, the others in global memory: entry i at
 // g[i + 1], so that the two children of an entry share a 32-byte sector.
 // Keys are the bits of the errors, which order as the non-negative errors
 // do (the subregions of a box whose error is not a number are never
-// compared: the box stops at its first bisection).
+// compared: the box stops at its first bisection).  kTop is odd, so the two
+// children of an entry lie on the same side of it.
 //
 // In global memory alone the pop took 3.5 k and the two pushes 2 k of the
 // 10 k cycles of a bisection late in a box of 2048.
+template <int kTop>
 struct SplitHeap {
-  static constexpr int kTop = 255;
-  static constexpr int kBytes = 3072;  // kTop keys and indices
+  static constexpr int kBytes = (kTop + 1) * 12;  // kTop keys and indices
   unsigned long long* key;
   int* id;
   P2HeapEnt* g;
@@ -454,8 +455,7 @@ struct SplitHeap {
     int x;
     load(--hn, k, x);
     int i = 0;
-    // children l and l + 1 lie on the same side of kTop (both odd); entry
-    // l + 1 may be past the end, and is then not used
+    // entry l + 1 may be past the end, and is then not used
     for (int l = 1; l < hn; l = 2 * i + 1) {
       unsigned long long kl, kr;
       int xl, xr;
@@ -527,8 +527,17 @@ constexpr int kSplitThreads = 128;
 template <int N, bool kWide>
 constexpr int kSplitLanes = N <= 2 ? 2 : (N <= 4 || !kWide) ? 4 : 8;
 constexpr long long kSplitWideBoxes = 1 << 16;
+// Heap entries in shared memory and blocks per SM: narrow groups have twice
+// the heaps, and gain from a fifth block (55.5 to 51.6 ms on the 2.0 M boxes;
+// the wide form lost 7% with the smaller heap and fewer registers).
 template <int K>
-constexpr int kSplitSmem = kSplitThreads / (2 * K) * detail::SplitHeap::kBytes;
+constexpr int kSplitTop = K == 8 ? 255 : 127;
+template <int K>
+constexpr int kSplitBlocks = K == 8 ? 4 : 5;
+template <int K>
+using SplitHeapOf = detail::SplitHeap<kSplitTop<K>>;
+template <int K>
+constexpr int kSplitSmem = kSplitThreads / (2 * K) * SplitHeapOf<K>::kBytes;
 __host__ __device__ inline int split_stride(int max_regions) { return (max_regions + 4) & ~1; }
 
 // Depth-first refinement with 2K lanes per box: the lower K lanes evaluate
@@ -542,7 +551,7 @@ __host__ __device__ inline int split_stride(int max_regions) { return (max_regio
 // 3.6 k for the children's sums, 1.7 k for their errors, the rest the heap
 // and the pool) and, with all lanes busy, by the pools' traffic through L2.
 template <int N, int K, class Src>
-__global__ void __launch_bounds__(kSplitThreads, 4) k_phase2_split(Src src, RuleTables T,
+__global__ void __launch_bounds__(kSplitThreads, (kSplitBlocks<K>)) k_phase2_split(Src src, RuleTables T,
                                                                    Phase2Args a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kGroup = 2 * K;
@@ -556,11 +565,11 @@ __global__ void __launch_bounds__(kSplitThreads, 4) k_phase2_split(Src src, Rule
   const long long group = ((long long)blockIdx.x * kSplitThreads + threadIdx.x) / kGroup;
   const int stride = split_stride(a.max_regions);
   P2Region<N>* pool = reinterpret_cast<P2Region<N>*>(a.slab) + group * stride;
-  extern __shared__ __align__(16) unsigned char split_dyn[];  // SplitHeap::kBytes a group
-  detail::SplitHeap heap;
+  extern __shared__ __align__(16) unsigned char split_dyn[];  // the groups' heap tops
+  SplitHeapOf<K> heap;
   heap.key = reinterpret_cast<unsigned long long*>(
-      split_dyn + (threadIdx.x / kGroup) * detail::SplitHeap::kBytes);
-  heap.id = reinterpret_cast<int*>(heap.key + detail::SplitHeap::kTop);
+      split_dyn + (threadIdx.x / kGroup) * SplitHeapOf<K>::kBytes);
+  heap.id = reinterpret_cast<int*>(heap.key + kSplitTop<K>);
   heap.g = a.heap + group * stride;
   bool more = true, have = false;
   int box = 0, k = 0, nreg = 0, used = 0, hn = 0;
