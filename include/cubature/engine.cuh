@@ -1026,7 +1026,7 @@ Workspace::LoopEntry* loop_graph(Workspace& ws, int sms) {
   ok = ok && kernel(arms[2], &n_ev, (const void*)k_loop_partials<Src>, sms * 16, 256, a_la, &n_part);
   ok = ok && kernel(body, &n_sw, (const void*)k_loop_tiles<Src>, sms * 4, 128, a_la, &n_tile);
   ok = ok && kernel(body, &n_tile, (const void*)k_loop_decide<Src>, sms * 16, 256, a_la, &n_dec);
-  ok = ok && kernel(body, &n_dec, (const void*)k_loop_scan<Src>, 1, 32, a_la, &n_scan);
+  ok = ok && kernel(body, &n_dec, (const void*)k_loop_scan<Src>, 1, kScanThreads, a_la, &n_scan);
   ok = ok && kernel(body, &n_scan, (const void*)k_loop_split<N, Src>, sms * 16, 256, a_la, &n_split);
   ok = ok && kernel(body, &n_split, (const void*)k_loop_advance<Src>, sms, 256, a_la, &n_adv);
   ok = ok && kernel(body, &n_adv, (const void*)k_loop_test<Src>, 1, 32, a_test, &n_test);
@@ -1439,7 +1439,7 @@ int run_batch(Workspace& ws, const Src& src, int nint, const double* epsrel,
       k_tiles<<<(unsigned)std::min<long long>((nblk + 3) / 4, sms * 4ll), 128, 0, s>>>(a);
     const unsigned db = (unsigned)std::max(1, std::min((nint + 7) / 8, sms * 16));
     k_decide<<<db, 256, 0, s>>>(a);
-    k_scan<<<1, 32, 0, s>>>(a);
+    k_scan<<<1, detail::kScanThreads, 0, s>>>(a);
     k_split<N><<<pb, 256, 0, s>>>(a);
     k_advance<<<(unsigned)std::max(1, std::min((nint + 255) / 256, sms)), 256, 0, s>>>(a);
     st.launches += 5 + (partials ? 1 : 0) + (nblk > 0 ? 1 : 0);

@@ -520,13 +520,16 @@ __device__ __forceinline__ void decide_warp(const EngineArgs& a, int k, int lane
   if (lane == 0) decide_integral(is, s0, s1, s2, s3, running, a);
 }
 
-// A single warp assigns the next segments (32-aligned) and the leftover
-// ranges of all integrals: an exclusive scan in integral order.
-__device__ __forceinline__ void scan_warp(const EngineArgs& a, int n_left_in, IterState* out,
-                                          int lane) {
+// One block of kScanThreads assigns the next segments (32-aligned) and the
+// leftover ranges of all integrals: an exclusive scan in integral order, an
+// integral per thread (a single warp took 10 us for 300 integrals).
+constexpr int kScanThreads = 512;
+__device__ __forceinline__ void scan_block(const EngineArgs& a, int n_left_in, IterState* out) {
+  __shared__ int wn[kScanThreads / 32], wl[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int carry_n = 0, carry_l = n_left_in, nrun = 0;
-  for (int base = 0; base < a.nint; base += 32) {
-    const int k = base + lane;
+  for (int base = 0; base < a.nint; base += kScanThreads) {
+    const int k = base + threadIdx.x;
     int vn = 0, vl = 0, r = 0;
     if (k < a.nint) {
       const IntegralState& is = a.ist[k];
@@ -544,19 +547,31 @@ __device__ __forceinline__ void scan_warp(const EngineArgs& a, int n_left_in, It
         il += tl;
       }
     }
+    if (lane == 31) {
+      wn[warp] = in;
+      wl[warp] = il;
+    }
+    nrun += __syncthreads_count(r);
+    int pn = carry_n, pl = carry_l;
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      if (w < warp) {
+        pn += wn[w];
+        pl += wl[w];
+      }
+      carry_n += wn[w];
+      carry_l += wl[w];
+    }
     if (k < a.nint) {
       IntegralState& is = a.ist[k];
-      is.next_start = carry_n + in - vn;
+      is.next_start = pn + in - vn;
       if (vl > 0) {
-        is.left_start = carry_l + il - vl;
+        is.left_start = pl + il - vl;
         is.left_count = vl;
       }
     }
-    carry_n += __shfl_sync(0xffffffffu, in, 31);
-    carry_l += __shfl_sync(0xffffffffu, il, 31);
-    nrun += __popc(__ballot_sync(0xffffffffu, r));
+    __syncthreads();  // wn and wl are read before the next pass writes them
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     IterState s;
     s.n = carry_n;
     s.n_running = nrun;
@@ -703,8 +718,10 @@ static __global__ void __launch_bounds__(256) k_decide(EngineArgs a) {
     detail::decide_warp(a, k, threadIdx.x & 31);
 }
 
-static __global__ void k_scan(EngineArgs a) {
-  detail::scan_warp(a, a.ctl->host.n_left, &a.ctl->host, threadIdx.x & 31);
+static __global__ void __launch_bounds__(detail::kScanThreads) k_scan(EngineArgs a) {
+  const int n_left = a.ctl->host.n_left;
+  __syncthreads();  // the block's last step overwrites it
+  detail::scan_block(a, n_left, &a.ctl->host);
 }
 
 template <int N>

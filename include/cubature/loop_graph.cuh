@@ -142,9 +142,11 @@ __global__ void __launch_bounds__(256) k_loop_decide(const LoopArgs<Src>* la) {
 }
 
 template <class Src>
-__global__ void k_loop_scan(const LoopArgs<Src>* la) {
+__global__ void __launch_bounds__(detail::kScanThreads) k_loop_scan(const LoopArgs<Src>* la) {
   const EngineArgs a = la->it;
-  detail::scan_warp(a, a.ctl->host.n_left, &a.ctl->host, threadIdx.x & 31);
+  const int n_left = a.ctl->host.n_left;
+  __syncthreads();  // the block's last step overwrites it
+  detail::scan_block(a, n_left, &a.ctl->host);
 }
 
 template <int N, class Src>

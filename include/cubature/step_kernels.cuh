@@ -70,19 +70,26 @@ static __global__ void k_step_count(long long n, const int* active, int* cnt) {
   }
 }
 
-// Split, pass 2: exclusive scan of the chunk counts (one block); writes the
-// child count 2m.
+// Split, pass 2: exclusive scan of the chunk counts (one block, 16 chunks a
+// thread and pass); writes the child count 2m.  One chunk a thread took 33 us
+// for the 31 k chunks of 1 M regions, a block-wide scan and its barriers per
+// 1024 of them.
+constexpr int kScanPer = 16;
 static __global__ void __launch_bounds__(1024) k_step_scan(long long nchunk, const int* cnt, int* excl,
                                                     long long* count_out) {
   __shared__ long long wsum[32];
-  __shared__ long long carry;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) carry = 0;
-  __syncthreads();
-  for (long long base = 0; base < nchunk; base += 1024) {
-    const long long c = base + tid;
-    const long long v = c < nchunk ? cnt[c] : 0;
-    long long incl = v;
+  long long carry = 0;
+  for (long long base = 0; base < nchunk; base += 1024 * kScanPer) {
+    const long long c0 = base + (long long)tid * kScanPer;
+    int v[kScanPer];
+    long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+      v[i] = c0 + i < nchunk ? cnt[c0 + i] : 0;
+      sum += v[i];
+    }
+    long long incl = sum;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const long long t = __shfl_up_sync(0xffffffffu, incl, off);
@@ -90,21 +97,21 @@ static __global__ void __launch_bounds__(1024) k_step_scan(long long nchunk, con
     }
     if (lane == 31) wsum[wid] = incl;
     __syncthreads();
-    if (wid == 0) {
-      long long w = wsum[lane];
+    long long w = wsum[lane];
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, w, off);
-        if (lane >= off) w += t;
-      }
-      wsum[lane] = w;
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long t = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) w += t;
     }
-    __syncthreads();
-    const long long wb = wid > 0 ? wsum[wid - 1] : 0;
-    if (c < nchunk) excl[c] = (int)(carry + wb + incl - v);
-    __syncthreads();
-    if (tid == 0) carry += wsum[31];
-    __syncthreads();
+    const long long before = __shfl_sync(0xffffffffu, w, wid > 0 ? wid - 1 : 0);
+    long long run = carry + (wid > 0 ? before : 0) + incl - sum;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+      if (c0 + i < nchunk) excl[c0 + i] = (int)run;
+      run += v[i];
+    }
+    carry += __shfl_sync(0xffffffffu, w, 31);
+    __syncthreads();  // wsum is read before the next pass writes it
   }
   if (tid == 0) *count_out = 2 * carry;
 }
@@ -177,15 +184,16 @@ static __global__ void __launch_bounds__(256) k_step_reduce(long long n, const d
   }
 }
 
-// Reduction, pass 2: one warp sums the block partials in a fixed order.
-static __global__ void k_step_reduce_final(int nblocks, const double* part, double* out) {
-  const int lane = threadIdx.x;
-  double s[4] = {0, 0, 0, 0};
-  for (int b = lane; b < nblocks; b += 32)
-    for (int q = 0; q < 4; ++q) s[q] += part[b * 4 + q];
-  for (int q = 0; q < 4; ++q) s[q] = warp_sum(s[q]);
-  if (lane == 0)
-    for (int q = 0; q < 4; ++q) out[q] = s[q];
+// Reduction, pass 2: a warp per sum, lane-strided over the block partials in a
+// fixed order (one warp for all four read 128 bytes a step and took 10 us).
+static __global__ void __launch_bounds__(128) k_step_reduce_final(int nblocks, const double* part,
+                                                                  double* out) {
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  double s = 0;
+#pragma unroll 8
+  for (int b = lane; b < nblocks; b += 32) s += part[b * 4 + q];
+  s = warp_sum(s);
+  if (lane == 0) out[q] = s;
 }
 
 }  // namespace cubature

@@ -544,7 +544,7 @@ int cub_reduce(long long n, const double* d_avg, const double* d_err, const int*
   const long long want = (n + 255) / 256;
   const int blocks = (int)std::max<long long>(1, std::min<long long>(want, kReduceBlocks));
   k_step_reduce<<<blocks, 256, 0, s>>>(n, d_avg, d_err, d_active, part);
-  k_step_reduce_final<<<1, 32, 0, s>>>(blocks, part, d_out);
+  k_step_reduce_final<<<1, 128, 0, s>>>(blocks, part, d_out);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "reduce kernel launch");
   return 0;
