@@ -724,14 +724,15 @@ inline void launch_eval(const Src& src, const RuleTables& T, const EngineArgs& a
 // List lengths from which the multi-launch rule kernel takes one lane and 8
 // lanes per region (below: 32).  Point by point, one lane needs a list that
 // fills the chip (512 regions an SM); a factored integrand (kFactored) costs
-// a tenth of that per region, and one lane is always the faster.
+// a tenth to a third of that per region, and one lane is the faster always or
+// from its kMinList on.
 struct EvalLanes {
   int k1_min, k8_min;
 };
 template <class Src>
 inline EvalLanes eval_lanes(int sms) {
-  if (detail::kFactored<detail::SourceFn<Src>>) return {0, 0};
-  return {sms * 512, sms * 64};
+  using F = detail::SourceFn<Src>;
+  return {detail::kFactored<F> ? detail::ThreadSums<F>::kMinList : sms * 512, sms * 64};
 }
 
 namespace detail {

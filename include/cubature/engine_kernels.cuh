@@ -31,6 +31,7 @@
 #include <utility>
 
 #include "integrands.cuh"
+#include "linear_sums.cuh"
 #include "region_rule.cuh"
 
 namespace cubature {

@@ -20,9 +20,11 @@
 //                   either way have the same bits,
 //   factor(t)       the axis' factor of the value,
 //   factor2(t, s)   factor(t) + factor(s),
-//   over(v, t)      v / factor(t),
-//   kNoise          a bound of the relative rounding error of the fold's
-//                   value and of the factors, with room to spare.
+//   inverse(t, c)   1 / c for the factor c of term t,
+//   noise(f0)       a bound of the rounding errors, relative to the values,
+//                   by which a difference of fold values near f0 and the same
+//                   difference formed from factors can disagree; three times
+//                   what the operations can add up to.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -80,9 +82,15 @@ struct Gaussian {
   __device__ __forceinline__ static double factor2(double t, double s) {
     return factor(t) + factor(s);
   }
-  __device__ __forceinline__ static double over(double v, double t) { return v / exp(-(t * t)); }
-  // the exponent is at most 745 where the value is not zero, summed in N steps
-  static constexpr double kNoise = 2e-13 * N;
+  __device__ __forceinline__ static double inverse(double, double c) { return 1 / c; }
+  // The exponent s of a value v = exp(-s) is summed in N roundings of at most
+  // s u (u = 2^-53) each, and v s is largest at the centre's s or below 1 / e;
+  // 8 u for the exponentials, sums and quotients.
+  __device__ __forceinline__ static double noise(double f0) {
+    const int e = (__double2hiint(f0) >> 20) & 0x7ff;  // f0 >= 2^(e - 1023)
+    const double s0 = e < 1022 ? 0.7 * (1023 - e) : 1.0;
+    return 3.4e-16 * (N * s0 + 8);
+  }
   __device__ __forceinline__ double operator()(const double* x) const {
     double s = start();
 #pragma unroll
@@ -172,8 +180,10 @@ struct ProductPeak {
     }
     return 1 / q + 1 / p;
   }
-  __device__ __forceinline__ static double over(double v, double q) { return v * q; }
-  static constexpr double kNoise = 4e-15 * (N + 6);
+  __device__ __forceinline__ static double inverse(double q, double) { return q; }
+  // N roundings of the product and the quotient, 8 of sums and factors; the
+  // terms are the same bits on both sides
+  __device__ __forceinline__ static double noise(double) { return 3.4e-16 * (N + 8); }
   __device__ __forceinline__ double operator()(const double* x) const {
     double den = start();
 #pragma unroll

@@ -756,16 +756,16 @@ static __device__ __noinline__ void scan_shift_warp(const EngineArgs& a, int n_l
   }
 }
 
-// Run by the warp that completed chunk c (owned by integral k).  Small
-// batches: sum the chunk; the warp that completes the last chunk of the
+// Run by the warp that completed chunk c (owned by integral k), whose partial
+// is formed here unless `summed`.  Small batches: the warp that completes the last chunk of the
 // list decides every integral and assigns the next list.  Large batches:
 // the warp that completes an integral's last chunk decides it, the one that
 // decides the last integral assigns the next list.
 static __device__ __noinline__ void after_chunk_warp(const EngineArgs& a, long long c, int k, int lane,
                                               const IterState& st, IterState* next,
-                                              int* chunk_int, int it, int g_next) {
+                                              int* chunk_int, int it, int g_next, bool summed) {
   __syncwarp();
-  chunk_partial_warp(a, c, lane);
+  if (!summed) chunk_partial_warp(a, c, lane);
   if (a.nint <= kSmallBatch) {
     unsigned last = 0;
     if (lane == 0) {
@@ -962,9 +962,79 @@ __device__ __forceinline__ void eval_step(const Src& src, const RuleTables& T, c
       // chunk's first slot always holds a region
       const long long c = slot / 32;
       const int kc = sm.owner[g] >= 0 ? sm.owner[g] : a.rid[c * 32];
-      after_chunk_warp(*sa, c, kc, lane, st, next, chunk_int, it, g_next);
+      after_chunk_warp(*sa, c, kc, lane, st, next, chunk_int, it, g_next, false);
     }
     __syncthreads();
+  }
+}
+
+// The eval step of factored integrands (kFactored) on lists longer than one
+// pass of the groups: a warp per chunk, a thread per slot.  The thread sets up
+// its region as a group does, writes it into the list and evaluates it from
+// there; the chunk's partial is summed on the spot.  A 4-D list of 15 k
+// regions took the groups of 32 lanes seven passes of 10 us.
+template <int N, class Src>
+__device__ __forceinline__ void eval_step_threads(const Src& src, const RuleTables& T,
+                                                  const EngineArgs& a, const PersistArgs& pa,
+                                                  const Parent& P, const Dest& D, const Stage& sg,
+                                                  int mode, const IterState& st, IterState* next,
+                                                  int* chunk_int, int it, int g_next,
+                                                  const EngineArgs* sa) {
+  const int lane = threadIdx.x & 31;
+  // consecutive chunks on different SMs
+  for (long long c = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x; c < st.n / 32;
+       c += (long long)gridDim.x * (blockDim.x / 32)) {
+    const long long slot = c * 32 + lane;
+    int k = -1;
+    double epsrel = 0, epsabs = 0;
+    if (mode == kSlotStored) {
+      k = a.rid[slot];
+      if (k >= 0) {
+        epsrel = a.ist[k].epsrel;
+        epsabs = a.ist[k].epsabs;
+      }
+    } else {
+      double L[N], H[N];
+      if (mode == kSlotGrid) {
+        k = initial_box<N>(slot, pa.divisions, pa.per_integral, pa.padded, pa.box, L, H);
+        if (k >= 0) {
+          epsrel = a.ist[k].epsrel;
+          epsabs = a.ist[k].epsabs;
+        }
+      } else {
+        const Origin o = lazy_origin(a, sg, slot);
+        k = o.k;
+        epsrel = o.epsrel;
+        epsabs = o.epsabs;
+        if (k >= 0) child_box<N>(P, o.par, o.side, L, H);
+      }
+      if (k >= 0) {
+#pragma unroll
+        for (int d = 0; d < N; ++d) {
+          D.lo[(long long)d * D.cap + slot] = L[d];
+          D.len[(long long)d * D.cap + slot] = H[d];
+        }
+      }
+      D.rid[slot] = k;
+    }
+    double av = 0, er = 0;
+    bool act = false;
+    if (k >= 0) {
+      RegionSums rs;
+      double jac;
+      const auto& f = source_view(src, k);
+      factored_sums<N, SourceFn<Src>>(f, ListBox{D.lo + slot, D.len + slot, D.cap}, T.ratio, rs, jac);
+      const RegionResult r = finish_region<N>(rs, T, jac, 0);
+      av = r.avg;
+      er = r.err;
+      act = er / max_err(av, epsrel, epsabs) > 1;
+      a.axis[slot] = r.axis;
+    }
+    __syncwarp();
+    store_chunk(a, c, lane, av, er, act);
+    // the chunk's first slot always holds a region
+    const int kc = __shfl_sync(0xffffffffu, k, 0);
+    after_chunk_warp(*sa, c, kc, lane, st, next, chunk_int, it, g_next, true);
   }
 }
 
@@ -1068,8 +1138,18 @@ __global__ void __launch_bounds__(256, 2) k_persistent(Src src, RuleTables T, Pe
 
     // smallest R (regions per block) that covers the list in one pass
     const long long per_block = (st.n + gridDim.x - 1) / gridDim.x;
+    bool threads = false;
+    if constexpr (detail::kFactored<detail::SourceFn<Src>>) {
+      // longer than a pass of the smallest groups (which beat the stand-alone
+      // rule's 32 lanes by a factor of two)
+      threads = per_block > p.max_r &&
+                st.n >= 2 * detail::ThreadSums<detail::SourceFn<Src>>::kMinList;
+      if (threads)
+        detail::eval_step_threads<N>(src, sm.tables, a, p, P, D, sg, mode, st, next, p.chunk_int,
+                                     it, g_it + 1, &sargs);
+    }
     const int r = per_block <= 1 ? 1 : (per_block <= 2 ? 2 : (per_block <= 4 ? 4 : 8));
-    switch (r < p.max_r ? r : p.max_r) {
+    if (!threads) switch (r < p.max_r ? r : p.max_r) {
       case 1:
         detail::eval_step<N, 256>(src, T, a, p, P, D, sg, mode, st, next, p.chunk_int, sm, it, g_it + 1, &sargs);
         break;

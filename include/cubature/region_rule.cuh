@@ -298,12 +298,13 @@ struct AxisChoice {
   double best = 0, second = 0, scale = 0;
   int axis = -1;
 
-  template <class F>
-  __device__ __forceinline__ void add(int d, double tc, double c, double s, double w,
+  // Axis d: centre factor c >= 0 and factor sums s, w at a1, a2, all of them
+  // times inv (> 0) over f0.
+  __device__ __forceinline__ void add(int d, double inv, double c, double s, double w,
                                       double ratio) {
     const double k = 2.0 * (1.0 - ratio);
-    const double v = F::over(fabs(fma(k, c, fma(ratio, s, -w))), tc);
-    scale = fmax(scale, F::over(fma(k, c, fma(ratio, s, w)), tc));
+    const double v = fabs(fma(k, c, fma(ratio, s, -w))) * inv;
+    scale = fmax(scale, fma(k, c, fma(ratio, fabs(s), fabs(w))) * inv);
     if (v > best) {
       second = best;
       best = v;
@@ -372,6 +373,41 @@ __device__ __noinline__ int exact_axis(const V& f, const Box& box, double ratio)
   return axis;
 }
 
+// The same choice from the values of the points themselves, for any functor:
+// the comparisons of region_point_sums, with the bits of f(x).
+template <int N, class F>
+__device__ __noinline__ int exact_axis_points(const F& f, const double (&L)[N],
+                                              const double (&H)[N], double ratio) {
+  double x[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = fma(0.5, H[i], L[i]);
+  const double base = __dmul_rn(__dmul_rn(f(x), 2.0), __dadd_rn(1.0, -ratio));
+  double best = 0;
+  int axis = -1;
+#pragma unroll 1
+  for (int d = 0; d < N; ++d) {
+    const double c = x[d];
+    double v[4];
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      const double g = k == 0   ? coef(kGenA1, false)
+                       : k == 1 ? coef(kGenA1, true)
+                       : k == 2 ? coef(kGenA2, false)
+                                : coef(kGenA2, true);
+      x[d] = fma(g, H[d], L[d]);
+      v[k] = f(x);
+    }
+    x[d] = c;
+    const double fd = fabs(__dadd_rn(__dadd_rn(base, __dmul_rn(ratio, __dadd_rn(v[0], v[1]))),
+                                     -__dadd_rn(v[2], v[3])));
+    if (fd > best) {
+      best = fd;
+      axis = d;
+    }
+  }
+  return axis;
+}
+
 // Set sums and fourth difference of one region by one thread, for
 // integrands that are products over the axes (AxisProductTrait).
 //
@@ -405,7 +441,7 @@ __device__ __forceinline__ void append_axis(const V& f, const Box& box, int d, d
   const double tc = ax.term(fma(0.5, Hd, Ld)), c = F::factor(tc);
   const double s = F::factor2(at(kGenA1, false), at(kGenA1, true));
   const double w = F::factor2(at(kGenA2, false), at(kGenA2, true));
-  ch.template add<F>(d, tc, c, s, w, ratio);
+  ch.add(d, F::inverse(tc, c), c, s, w, ratio);
   poly.append(c, s, w, F::factor2(at(kGenA3, false), at(kGenA3, true)),
               F::factor2(at(kGenA4, false), at(kGenA4, true)),
               F::factor2(at(kGenL, false), at(kGenL, true)));
@@ -422,7 +458,7 @@ __device__ __forceinline__ void axis_product_sums(const V& f, const Box& box, do
   for (int d = 0; d < N; ++d) append_axis<F>(f, box, d, ratio, poly, ch, jac);
   poly.store(out);
   out.best = ch.best;
-  out.axis = ch.sure(F::kNoise, poly.z) ? ch.axis : exact_axis<N, F>(f, box, ratio);
+  out.axis = ch.sure(F::noise(poly.z), poly.z) ? ch.axis : exact_axis<N, F>(f, box, ratio);
 }
 
 // axis_product_sums with the axes dealt to the K lanes of a group (lane j:
@@ -449,7 +485,7 @@ __device__ __forceinline__ void axis_split_sums(const V& f, const Box& box, int 
 #pragma unroll
   for (int k = 0; k < kNumSets; ++k) out.S[k] = __shfl_sync(mask, out.S[k], 0, K);
   out.best = ch.best;
-  out.axis = ch.sure(F::kNoise, out.S[0]) ? ch.axis : exact_axis<N, F>(f, box, ratio);
+  out.axis = ch.sure(F::noise(out.S[0]), out.S[0]) ? ch.axis : exact_axis<N, F>(f, box, ratio);
 }
 
 // A box in an SoA region list.
@@ -462,38 +498,56 @@ struct ListBox {
 };
 
 // Functors with an evaluator of their own for one region by one thread:
-// ThreadSums<F>::run(f, L, H, ratio, out).
+// ThreadSums<F>::run(f, L, H, ratio, out).  kMinList: the list length from
+// which it beats several lanes per region.
 template <class F>
 struct ThreadSums {
   static constexpr bool value = false;
+  static constexpr int kMinList = 0;
 };
 
 // One thread per region has a form that shares work between the rule's
-// points: then it is the faster one for every list length that the
-// multi-launch driver sees, else only for lists that fill the chip.
+// points: it is then the faster one for every list length, or from kMinList
+// on; else only for lists that fill the chip.
 template <class F>
 constexpr bool kFactored = AxisProductTrait<F>::value || ThreadSums<F>::value;
+
+// The sums of one region of a factored integrand by one thread, and its
+// volume.
+template <int N, class F, class V, class Box>
+__device__ __forceinline__ void factored_sums(const V& f, const Box& box, double ratio,
+                                              RegionSums& out, double& jac) {
+  if constexpr (AxisProductTrait<F>::value) {
+    axis_product_sums<N, F>(f, box, ratio, out, jac);
+  } else {
+    double L[N], H[N];
+    jac = 1;
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      L[d] = box.lo(d);
+      H[d] = box.len(d);
+      jac = __dmul_rn(jac, H[d]);
+    }
+    ThreadSums<F>::run(f, L, H, ratio, out);
+  }
+}
 
 // The sums of one region by one thread, and its volume.
 template <int N, class F, class V, class Box>
 __device__ __forceinline__ void thread_sums(const V& f, const Box& box, const ItemTable<N>& tab,
                                             double ratio, RegionSums& out, double& jac) {
-  if constexpr (AxisProductTrait<F>::value) {
-    axis_product_sums<N, F>(f, box, ratio, out, jac);
+  if constexpr (kFactored<F>) {
+    factored_sums<N, F>(f, box, ratio, out, jac);
   } else {
     double L[N], H[N];
+    jac = 1;
 #pragma unroll
     for (int d = 0; d < N; ++d) {
       L[d] = box.lo(d);
       H[d] = box.len(d);
+      jac = __dmul_rn(jac, H[d]);
     }
-    if constexpr (ThreadSums<F>::value)
-      ThreadSums<F>::run(f, L, H, ratio, out);
-    else
-      region_point_sums<N, 1>(f, L, H, 0, tab, ratio, out);
-    jac = 1;
-#pragma unroll
-    for (int d = 0; d < N; ++d) jac = __dmul_rn(jac, H[d]);
+    region_point_sums<N, 1>(f, L, H, 0, tab, ratio, out);
   }
 }
 

@@ -11,7 +11,7 @@ namespace cubature {
 // warp).  Point by point: when the list fills the chip.
 template <class F>
 inline long long rule_thread_min(int sms) {
-  return detail::kFactored<F> ? 0 : sms * 512ll;
+  return detail::kFactored<F> ? detail::ThreadSums<F>::kMinList : sms * 512ll;
 }
 
 // Rule + classification over one integral's SoA list (INTEGRATE_GPU_PHASE1,

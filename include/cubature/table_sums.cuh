@@ -21,6 +21,7 @@ namespace detail {
 template <>
 struct ThreadSums<Table7<7>> {
   static constexpr bool value = true;
+  static constexpr int kMinList = 0;
   __device__ __forceinline__ static void run(const Table7<7>& f, const double (&L)[7], const double (&H)[7],
                                               double ratio, RegionSums& out) {
     auto kernel = [&](double r) { return f.kernel(r); };

@@ -1,8 +1,9 @@
 """Kernels that share work between the points of a region, at the sizes and
 inputs where they can go wrong, against the point-by-point oracle.
 
-Integrands that are products over the axes, and the 7-D table integrand, are
-evaluated by one thread per region from per-axis (per-group) factors.  Values
+Integrands that are products over the axes, those that depend on a sum over
+the axes, and the 7-D table integrand are evaluated by one thread per region
+from per-axis (per-group) quantities.  Values
 and errors are sums of the same terms in another order: the tolerances are
 those of tests/test_gpu_parity.py (1e-13 of the L1 magnitude of the rule sum
 for the value, 1e-12 for the error), the split axes identical where the
@@ -38,7 +39,41 @@ def test_product_rule_list_lengths(cub, oracle, ctx, family, n, m):
     compare_regions(o, _eval(cub, family, n, a, u, lo, ln), (family, n, m))
 
 
+@pytest.mark.parametrize("family", ["corner_peak", "continuous"])
+@pytest.mark.parametrize("n", range(2, 9))
+@pytest.mark.parametrize("m", [33, 12321])
+def test_sum_rule_list_lengths(cub, oracle, ctx, family, n, m):
+    """12321 regions are past the length from which every family takes one
+    thread per region, and no multiple of a block."""
+    rng = np.random.default_rng(200 * n + m)
+    a, u = FAMILY_PARAMS[family](n, rng)
+    level = rng.binomial(6, 0.5, (n, m))
+    ln = np.ldexp(1.0, -level)
+    lo = np.floor(rng.random((n, m)) / ln) * ln
+    o = oracle.Rule(n).phase1_eval(oracle.make_integrand(family, n, a, u), lo, ln, 1e-4, 1e-12)
+    compare_regions(o, _eval(cub, family, n, a, u, lo, ln), (family, n, m))
+
+
+@pytest.mark.parametrize("family,a,u", [
+    ("continuous", [-2.0, 3.0, 1.0, -0.5], [0.3, 0.6, 0.5, 0.4]),  # factors above 1
+    ("continuous", [2.0, 0.0, 1.0, 0.5], [0.3, 0.6, 0.5, 0.4]),    # ties, an idle axis
+    ("corner_peak", [3.0, -0.2, 0.0, 1.0], [0.0] * 4),             # signs mixed, an idle axis
+    ("corner_peak", [9.0, 7.0, 11.0, 8.0], [0.0] * 4),
+])
+def test_sum_rule_unusual_parameters(cub, ctx, family, a, u):
+    """Against 32 lanes point by point in the engine: the same splits."""
+    f = cub.Integrand(family, 4, a, u)
+    opt = dict(policy=cub.POLICY_BREADTH, persistent=False)
+    one = ctx.integrate(f, 1e-7, 1e-12, cub.options(lanes=1, **opt))
+    many = ctx.integrate(f, 1e-7, 1e-12, cub.options(lanes=32, **opt))
+    assert one.nregions == many.nregions and one.iterations == many.iterations
+    assert one.status == many.status
+    assert math.isclose(one.integral, many.integral, rel_tol=1e-12)
+
+
 @pytest.mark.parametrize("family,n,a,eps", [("gaussian", 5, 5.0, 1e-5), ("gaussian", 3, 6.0, 1e-9),
+                                            ("corner_peak", 4, 0.5, 1e-10),
+                                            ("continuous", 3, 4.0, 1e-9),
                                             ("product_peak", 2, 20.0, 1e-10),
                                             ("product_peak", 6, 4.0, 1e-5)])
 def test_tied_axes_split_as_point_by_point(cub, ctx, family, n, a, eps):
