@@ -95,6 +95,17 @@ def flops_per_region(family: str, n: int) -> float:
     return npoints(n) * per_eval + 5 * n + 3 * 9 * 3 + 8
 
 
+# FP64 flops of a region through the thread-per-region evaluators, which form
+# the rule's sums from per-axis (per-group) factors (a division or a
+# transcendental = 1): 11 terms, 11 factors and the set polynomials per axis;
+# for the table integrand 153 kernel, 33 table and 11 spline values.
+FACTORED = {
+    "product_peak": lambda n: 155 * n + 5 * n + 240,
+    "gaussian": lambda n: 150 * n + 5 * n + 240,
+    "table7": lambda n: 2400,
+}
+
+
 def product_peak_params(n: int, count: int):
     import numpy as np
 
@@ -742,14 +753,17 @@ def main() -> int:
     persist_flops = ml_flops = p2_flops = 0.0
     for (fam, n), (pk_r, ml_r, p2_r) in split.items():
         persist_flops += pk_r * flops_per_region(fam, n) * args.steps
-        ml_flops += ml_r * flops_per_region(fam, n) * args.steps
-        p2_flops += p2_r * flops_per_region(fam, n) * args.steps
+        factored = FACTORED.get(fam, lambda n: flops_per_region(fam, n))(n)
+        ml_flops += ml_r * factored * args.steps
+        p2_flops += p2_r * args.steps * (factored if fam != "table7" else
+                                         flops_per_region(fam, n))
     pk_name = "k_replicated" if st.get("replicated_launches", 0) >= max(
         1, st["persistent_launches"] - st.get("replicated_launches", 0)) else "k_persistent"
     kernels = {
         pk_name: (persist_flops, st["ms_persistent"]),
         "k_eval": (ml_flops, st["ms_eval"]),
-        "k_phase2": (p2_flops, st["ms_phase2"]),
+        "k_phase2_split" if any(f in ("product_peak", "gaussian") for f, _ in split)
+        else "k_phase2": (p2_flops, st["ms_phase2"]),
     }
     dom = max(kernels, key=lambda k: kernels[k][1])
     dom_flops, dom_ms = kernels[dom]

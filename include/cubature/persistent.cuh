@@ -757,15 +757,16 @@ static __device__ __noinline__ void scan_shift_warp(const EngineArgs& a, int n_l
 }
 
 // Run by the warp that completed chunk c (owned by integral k), whose partial
-// is formed here unless `summed`.  Small batches: the warp that completes the last chunk of the
+// is formed here unless kSummed.  Small batches: the warp that completes the last chunk of the
 // list decides every integral and assigns the next list.  Large batches:
 // the warp that completes an integral's last chunk decides it, the one that
 // decides the last integral assigns the next list.
+template <bool kSummed>
 static __device__ __noinline__ void after_chunk_warp(const EngineArgs& a, long long c, int k, int lane,
                                               const IterState& st, IterState* next,
-                                              int* chunk_int, int it, int g_next, bool summed) {
+                                              int* chunk_int, int it, int g_next) {
   __syncwarp();
-  if (!summed) chunk_partial_warp(a, c, lane);
+  if constexpr (!kSummed) chunk_partial_warp(a, c, lane);
   if (a.nint <= kSmallBatch) {
     unsigned last = 0;
     if (lane == 0) {
@@ -962,7 +963,7 @@ __device__ __forceinline__ void eval_step(const Src& src, const RuleTables& T, c
       // chunk's first slot always holds a region
       const long long c = slot / 32;
       const int kc = sm.owner[g] >= 0 ? sm.owner[g] : a.rid[c * 32];
-      after_chunk_warp(*sa, c, kc, lane, st, next, chunk_int, it, g_next, false);
+      after_chunk_warp<false>(*sa, c, kc, lane, st, next, chunk_int, it, g_next);
     }
     __syncthreads();
   }
@@ -1034,7 +1035,7 @@ __device__ __forceinline__ void eval_step_threads(const Src& src, const RuleTabl
     store_chunk(a, c, lane, av, er, act);
     // the chunk's first slot always holds a region
     const int kc = __shfl_sync(0xffffffffu, k, 0);
-    after_chunk_warp(*sa, c, kc, lane, st, next, chunk_int, it, g_next, true);
+    after_chunk_warp<true>(*sa, c, kc, lane, st, next, chunk_int, it, g_next);
   }
 }
 
