@@ -546,7 +546,7 @@ __host__ __device__ inline int split_stride(int max_regions) { return (max_regio
 // done gives its lanes to the next box of the work counter.
 //
 // Against a warp per box with 16 lanes per child (k_phase2), 2.0 M boxes of
-// 6-D product peaks (60 M subregions) went from 299 to 55 ms on a B200.
+// 6-D product peaks (60 M subregions) went from 299 to 52 ms on a B200.
 // Bound by the latency of a bisection (10 k cycles when few boxes are left:
 // 3.6 k for the children's sums, 1.7 k for their errors, the rest the heap
 // and the pool) and, with all lanes busy, by the pools' traffic through L2.
