@@ -461,19 +461,29 @@ __device__ __forceinline__ void axis_product_sums(const V& f, const Box& box, do
   out.axis = ch.sure(F::noise(poly.z), poly.z) ? ch.axis : exact_axis<N, F>(f, box, ratio);
 }
 
-// axis_product_sums with the axes dealt to the K lanes of a group (lane j:
-// axes j, j + K, ...), for chains of dependent regions, where the latency of
-// one region counts: a lane evaluates its axes' factors, and the lanes'
-// polynomials are joined by shuffles.  Every lane of the group (mask, K
+// axis_product_sums with the axes dealt to the K lanes of a group (lane j: a
+// run of neighbouring axes), for chains of dependent regions, where the
+// latency of one region counts: a lane evaluates its axes' factors, and the
+// lanes' polynomials are joined by shuffles.  Every lane of the group (mask, K
 // aligned lanes) gets the sums.
+//
+// The sums have the same bits for every K that gives a lane one axis or two:
+// appending an axis to another is joining the two (the terms that append
+// leaves out are products with zeros), and lanes of two axes start with the
+// pairs that lanes of one axis join first.  So a box is refined the same way
+// whichever K its call takes.  (With axes j and j + K on lane j the last bits
+// changed with K.)
 template <int N, int K, class F, class V, class Box>
 __device__ __forceinline__ void axis_split_sums(const V& f, const Box& box, int j, unsigned mask,
                                                 double ratio, RegionSums& out, double& jac) {
   AxisPoly poly;
   AxisChoice ch;
   jac = 1;
+  constexpr int kPer = (N + K - 1) / K;
+  static_assert(kPer <= 2, "the joins' order depends on K");
+  const int d1 = (j + 1) * kPer < N ? (j + 1) * kPer : N;
 #pragma unroll 1
-  for (int d = j; d < N; d += K) append_axis<F>(f, box, d, ratio, poly, ch, jac);
+  for (int d = j * kPer; d < d1; ++d) append_axis<F>(f, box, d, ratio, poly, ch, jac);
   __syncwarp(mask);
 #pragma unroll
   for (int off = 1; off < K; off <<= 1) {
