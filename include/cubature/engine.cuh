@@ -32,6 +32,7 @@
 #include "persistent.cuh"
 #include "loop_graph.cuh"
 #include "phase2_kernels.cuh"
+#include "pool_size.hpp"
 #include "replicated.cuh"
 #include "rule9.hpp"
 
@@ -108,7 +109,7 @@ inline const char* state_name(int s) {
   return "?";
 }
 
-inline long long auto_max_slots(int ndim, int policy);
+inline long long auto_max_slots(int ndim, int policy, size_t reusable);
 
 class Workspace {
  public:
@@ -162,6 +163,7 @@ class Workspace {
     for (auto& v : auto_slots_) v = 0;
     nint_cap_ = 0;
     slab_bytes_ = 0;
+    pool_bound_ = PoolBound();
     ndim_ = 0;
   }
 
@@ -260,8 +262,8 @@ class Workspace {
     double *nlo[2] = {nullptr, nullptr}, *nlen[2] = {nullptr, nullptr};
     int* nrid[2] = {nullptr, nullptr};
     for (int b = 0; b < 2; ++b) {
-      if (!alloc(&nlo[b], sizeof(double) * ndim * ncap) ||
-          !alloc(&nlen[b], sizeof(double) * ndim * ncap) || !alloc(&nrid[b], sizeof(int) * ncap))
+      if (!alloc_list(&nlo[b], sizeof(double) * ndim * ncap) ||
+          !alloc_list(&nlen[b], sizeof(double) * ndim * ncap) || !alloc_list(&nrid[b], sizeof(int) * ncap))
         return false;
     }
     if (keep > 0 && ndim == ndim_) {
@@ -287,14 +289,14 @@ class Workspace {
     }
     free_scratch();
     const long long nchunk = ncap / 32 + 1;
-    if (!alloc(&avg, sizeof(double) * ncap) || !alloc(&err, sizeof(double) * ncap) ||
-        !alloc(&axis, sizeof(int) * ncap) || !alloc(&active, sizeof(int) * ncap) ||
-        !alloc(&part, sizeof(ChunkPartial) * nchunk) || !alloc(&chunk_excl, sizeof(int) * nchunk) ||
-        !alloc(&tile, sizeof(TileSum) * (nchunk / kTileChunks + 1)) ||
-        !alloc(&chunk_cnt, sizeof(unsigned) * nchunk) || !alloc(&axis_alt, sizeof(int) * ncap) ||
-        !alloc(&excl_alt, sizeof(int) * nchunk) || !alloc(&cmask, sizeof(unsigned) * 2 * nchunk) ||
-        !alloc(&chunk_int, sizeof(int) * nchunk) || !alloc(&avg_alt, sizeof(double) * ncap) ||
-        !alloc(&err_alt, sizeof(double) * ncap))
+    if (!alloc_list(&avg, sizeof(double) * ncap) || !alloc_list(&err, sizeof(double) * ncap) ||
+        !alloc_list(&axis, sizeof(int) * ncap) || !alloc_list(&active, sizeof(int) * ncap) ||
+        !alloc_list(&part, sizeof(ChunkPartial) * nchunk) || !alloc_list(&chunk_excl, sizeof(int) * nchunk) ||
+        !alloc_list(&tile, sizeof(TileSum) * (nchunk / kTileChunks + 1)) ||
+        !alloc_list(&chunk_cnt, sizeof(unsigned) * nchunk) || !alloc_list(&axis_alt, sizeof(int) * ncap) ||
+        !alloc_list(&excl_alt, sizeof(int) * nchunk) || !alloc_list(&cmask, sizeof(unsigned) * 2 * nchunk) ||
+        !alloc_list(&chunk_int, sizeof(int) * nchunk) || !alloc_list(&avg_alt, sizeof(double) * ncap) ||
+        !alloc_list(&err_alt, sizeof(double) * ncap))
       return false;
     if (!ck(cudaMemsetAsync(chunk_cnt, 0, sizeof(unsigned) * nchunk, s))) return false;
     cap_ = ncap;
@@ -319,8 +321,8 @@ class Workspace {
     double *nlo = nullptr, *nlen = nullptr;
     int* nrid = nullptr;
     LeftoverResult* nres = nullptr;
-    if (!alloc(&nlo, sizeof(double) * ndim * ncap) || !alloc(&nlen, sizeof(double) * ndim * ncap) ||
-        !alloc(&nrid, sizeof(int) * ncap) || !alloc(&nres, sizeof(LeftoverResult) * ncap))
+    if (!alloc_list(&nlo, sizeof(double) * ndim * ncap) || !alloc_list(&nlen, sizeof(double) * ndim * ncap) ||
+        !alloc_list(&nrid, sizeof(int) * ncap) || !alloc_list(&nres, sizeof(LeftoverResult) * ncap))
       return false;
     if (keep > 0 && ndim == left_ndim_) {
       for (int d = 0; d < ndim; ++d) {
@@ -348,11 +350,12 @@ class Workspace {
   }
 
   // Automatic region capacity for (ndim, policy), measured once (free
-  // device memory) and kept until release().
+  // device memory, the second phase's pools included: the lists may take
+  // theirs) and kept until release().
   long long auto_slots(int ndim, int policy) {
     const int i = 2 * ndim + (policy == kPolicyReference ? 1 : 0);
-    if (ndim < 0 || ndim > kMaxDim) return auto_max_slots(ndim, policy);
-    if (!auto_slots_[i]) auto_slots_[i] = auto_max_slots(ndim, policy);
+    if (ndim < 0 || ndim > kMaxDim) return auto_max_slots(ndim, policy, pool_bytes());
+    if (!auto_slots_[i]) auto_slots_[i] = auto_max_slots(ndim, policy, pool_bytes());
     return auto_slots_[i];
   }
 
@@ -434,14 +437,24 @@ class Workspace {
 
   bool reserve_slab(size_t bytes, size_t heap_ints) {
     if (bytes <= slab_bytes_ && heap_ints <= heap_ints_) return true;
-    free_buf(slab);
-    free_buf(heap);
-    slab_bytes_ = heap_ints_ = 0;
+    drop_pool();
     if (!alloc(&slab, bytes) || !alloc(&heap, sizeof(int) * heap_ints)) return false;
     slab_bytes_ = bytes;
     heap_ints_ = heap_ints;
     return true;
   }
+
+  // The second phase's pools: their bytes, and how many more they may take.
+  size_t pool_bytes() const { return slab_bytes_ + sizeof(int) * heap_ints_; }
+  const PoolBound& pool_bound() {
+    if (!pool_bound_.share) {
+      size_t free_b = 0, total_b = 0;
+      if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
+      pool_bound_.share = std::max<size_t>((free_b + pool_bytes()) / 8, 1);
+    }
+    return pool_bound_;
+  }
+  void pool_refused(size_t bytes) { pool_bound_.refused = std::min(pool_bound_.refused, bytes); }
 
   bool ck(cudaError_t e) {
     if (e != cudaSuccess) {
@@ -615,6 +628,21 @@ class Workspace {
     bytes_ += bytes;
     return true;
   }
+  // A region or leftover list's buffer.  The second phase, whose pools hold
+  // nothing between calls, gives them up where memory is short.
+  template <class T>
+  bool alloc_list(T** p, size_t bytes) {
+    if (alloc(p, bytes)) return true;
+    if (!slab && !heap) return false;
+    cudaGetLastError();
+    drop_pool();
+    return alloc(p, bytes);
+  }
+  void drop_pool() {
+    free_buf(slab);
+    free_buf(heap);
+    slab_bytes_ = heap_ints_ = 0;
+  }
   template <class T>
   void free_buf(T*& p) {
     if (!p) return;
@@ -635,6 +663,7 @@ class Workspace {
   int ndim_ = 0, left_ndim_ = 0;
   int nint_cap_ = 0;
   size_t slab_bytes_ = 0, heap_ints_ = 0;
+  PoolBound pool_bound_;
   size_t box_cap_ = 0;
   void* ctl_block_ = nullptr;
   void* host_block_ = nullptr;
@@ -698,10 +727,12 @@ inline int sm_count(int device) {
 // Region-list capacity when the caller leaves it to the library: the slots
 // that fit in 40% of the device's free memory (two lists of FP64 bounds plus
 // per-slot results and chunk scratch, and leftover boxes under the reference
-// policy), between 2^20 and 2^30.
-inline long long auto_max_slots(int ndim, int policy) {
+// policy), between 2^20 and 2^30.  reusable: bytes the caller holds that count
+// as free.
+inline long long auto_max_slots(int ndim, int policy, size_t reusable) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b == 0) return 1ll << 26;
+  free_b += reusable;
   double per_slot = 2.0 * (16.0 * ndim + 4) + 28 + 64.0 / 32;
   if (policy == kPolicyReference) per_slot += 2.0 * (16.0 * ndim + 4 + 24);
   const double slots = 0.4 * (double)free_b / per_slot;
@@ -1103,8 +1134,9 @@ struct Phase2Launch {
   template <int K>
   bool reserve_split(Workspace& ws, const Options& opt, long long boxes, int sms) {
     // a pool and a heap per box in flight: as many boxes as the chip holds,
-    // fewer when memory is short
+    // fewer when memory is short (pool_blocks)
     constexpr int kBoxes = kSplitThreads / (2 * K);  // per block
+    constexpr int kWarpBoxes = 12;                   // per SM, a warp per box
     int per_sm = 0;
     if (!ws.ck(cudaFuncSetAttribute(k_phase2_split<N, K, Src>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1112,15 +1144,18 @@ struct Phase2Launch {
         !ws.ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &per_sm, k_phase2_split<N, K, Src>, kSplitThreads, kSplitSmem<K>)))
       return false;
-    blocks = std::min<long long>((long long)sms * std::max(1, per_sm),
-                                 (boxes + kBoxes - 1) / kBoxes);
-    const size_t stride = (size_t)split_stride(opt.phase2_max_regions);
-    for (blocks = std::max<long long>(blocks, 1);; blocks /= 2) {
-      const size_t n = (size_t)blocks * kBoxes * stride;
+    const long long want = std::max<long long>(
+        1, std::min<long long>((long long)sms * std::max(1, per_sm), (boxes + kBoxes - 1) / kBoxes));
+    const size_t block_entries = (size_t)kBoxes * split_stride(opt.phase2_max_regions);
+    const size_t block_bytes = block_entries * (sizeof(P2Region<N>) + sizeof(P2HeapEnt));
+    for (;;) {
+      blocks = pool_blocks(want, (long long)sms * kWarpBoxes / kBoxes, block_bytes, ws.pool_bound());
+      const size_t n = (size_t)blocks * block_entries;
       if (ws.reserve_slab(sizeof(P2Region<N>) * n, n * (sizeof(P2HeapEnt) / sizeof(int))))
         return true;
       cudaGetLastError();
       if (blocks == 1) return false;
+      ws.pool_refused((size_t)blocks * block_bytes);
     }
   }
 
