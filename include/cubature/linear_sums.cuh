@@ -6,9 +6,7 @@
 //   corner peak   with the argument b at the centre and increments
 //                 t_d = a_d g H_d the points pair up as (b + s)^-(N+1) +
 //                 (b - s)^-(N+1), one division per pair;
-//   continuous    a product over the axes, exp(-a_d |x_d - u_d|) each, for
-//                 a_d >= 0 (a factor above 1 could overflow where the value
-//                 does not: then point by point).
+//   continuous    a product over the axes, exp(-a_d |x_d - u_d|) each.
 // The split axis comes from these sums where they tell the axes apart by more
 // than the rounding, else from the points (exact_axis_points).
 //
@@ -138,10 +136,16 @@ struct ThreadSums<CornerPeak<N>> {
 };
 
 // 11 N exponentials instead of one per point (for 2 dimensions 22 against 33).
+//
+// With coefficients of both signs a product of some axes' factors can leave
+// the range of a double where the value does not; with exponents that add up to
+// less than kRange over the box none does.  Beyond it (values of 1e260, or
+// their reciprocals, inside one box) the region is evaluated point by point.
 template <int N>
 struct ThreadSums<Continuous<N>> {
   static constexpr bool value = true;
   static constexpr int kMinList = 0;
+  static constexpr double kRange = 600;
   __device__ __noinline__ static void by_points(const Continuous<N>& f, const double (&L)[N],
                                                 const double (&H)[N], double ratio,
                                                 RegionSums& out) {
@@ -151,12 +155,18 @@ struct ThreadSums<Continuous<N>> {
   }
   __device__ __forceinline__ static void run(const Continuous<N>& f, const double (&L)[N],
                                              const double (&H)[N], double ratio, RegionSums& out) {
-    bool ok = true;
+    bool decays = true;
 #pragma unroll
-    for (int i = 0; i < N; ++i) ok = ok && f.a[i] >= 0;
-    if (!ok) {
-      by_points(f, L, H, ratio, out);
-      return;
+    for (int i = 0; i < N; ++i) decays = decays && f.a[i] >= 0;
+    double reach = 0;  // largest sum of the exponents' magnitudes
+    if (!decays) {
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        reach = fma(fabs(f.a[i]), fmax(fabs(L[i] - f.u[i]), fabs(L[i] + H[i] - f.u[i])), reach);
+      if (!(reach < kRange)) {
+        by_points(f, L, H, ratio, out);
+        return;
+      }
     }
     AxisPoly poly;
     AxisChoice ch;
@@ -177,9 +187,10 @@ struct ThreadSums<Continuous<N>> {
     }
     poly.store(out);
     out.best = ch.best;
-    // as Gaussian::noise: the exponent of a value is summed in N roundings
+    // as Gaussian::noise: the exponent of a value is summed in N roundings (of
+    // at most `reach` each where its terms have both signs)
     const int e = (__double2hiint(poly.z) >> 20) & 0x7ff;
-    const double s0 = e < 1022 ? 0.7 * (1023 - e) : 1.0;
+    const double s0 = !decays ? reach : e < 1022 ? 0.7 * (1023 - e) : 1.0;
     out.axis = ch.sure(kRound3 * (2 * N * s0 + 8), poly.z) ? ch.axis
                                                            : exact_axis_points<N>(f, L, H, ratio);
   }
