@@ -95,6 +95,16 @@ def flops_per_region(family: str, n: int) -> float:
     return npoints(n) * per_eval + 5 * n + 3 * 9 * 3 + 8
 
 
+def pair_flops(n: int) -> float:
+    """FP64 flops of corner peak's pairs of points: per pair the increment (2),
+    two arguments, two powers by squaring, their sum and product, the division
+    and the set's sum."""
+    from cubature import npoints
+
+    power = (n + 1).bit_length() - 1 + bin(n + 1).count("1") - 1
+    return (npoints(n) - 1) / 2 * (2 + 2 + 2 * power + 3 + 1) + 5 * n + 240
+
+
 # FP64 flops of a region through the thread-per-region evaluators, which form
 # the rule's sums from per-axis (per-group) factors (a division or a
 # transcendental = 1): 11 terms, 11 factors and the set polynomials per axis;
@@ -102,8 +112,32 @@ def flops_per_region(family: str, n: int) -> float:
 FACTORED = {
     "product_peak": lambda n: 155 * n + 5 * n + 240,
     "gaussian": lambda n: 150 * n + 5 * n + 240,
+    "corner_peak": pair_flops,
     "table7": lambda n: 2400,
 }
+
+
+def kernel_flops(split: dict, steps: int, persistent: str):
+    """FP64 flops of `steps` steps in the persistent kernel (named by
+    `persistent`), the multi-launch rule kernel and the second phase, from
+    {(family, ndim): regions of a step in each}.
+
+    k_replicated evaluates points.  k_persistent takes the factored evaluators
+    on its longer lists; how many of its regions those were is not counted, so
+    it has no flop count (None) when a family that has one ran there.
+    """
+    p = ml = p2 = 0.0
+    for (fam, n), (p_r, ml_r, p2_r) in split.items():
+        points = flops_per_region(fam, n)
+        factored = FACTORED[fam](n) if fam in FACTORED else points
+        if persistent == "k_persistent" and fam in FACTORED and p_r:
+            p = None
+        elif p is not None:
+            p += p_r * points * steps
+        ml += ml_r * factored * steps
+        # the second phase factors products over the axes only
+        p2 += p2_r * (factored if fam in ("product_peak", "gaussian") else points) * steps
+    return p, ml, p2
 
 
 def product_peak_params(n: int, count: int):
@@ -743,25 +777,15 @@ def main() -> int:
     value = good * args.steps / (dev_ms / 1e3)
     e2e_value = good * args.steps / (wall / 1e3)
 
-    # roofline of the dominant kernel (FP64-bound rule evaluation).  The
-    # regions are split between the persistent kernel (short lists) and the
-    # multi-launch rule kernel (long lists); each gets its own share of the
-    # algorithmic flops (per-region flops x regions it evaluated).
     # Roofline of the dominant kernel (FP64-bound rule evaluation).  Each
     # kernel gets the algorithmic flops of the regions it evaluated, per
     # (family, ndim): the split of every integrand's regions between the
     # persistent kernels and the multi-launch rule kernel is taken from one
     # untimed pass with the counters read after each call (the split is the
     # same every step).
-    persist_flops = ml_flops = p2_flops = 0.0
-    for (fam, n), (pk_r, ml_r, p2_r) in split.items():
-        persist_flops += pk_r * flops_per_region(fam, n) * args.steps
-        factored = FACTORED.get(fam, lambda n: flops_per_region(fam, n))(n)
-        ml_flops += ml_r * factored * args.steps
-        p2_flops += p2_r * args.steps * (factored if fam != "table7" else
-                                         flops_per_region(fam, n))
     pk_name = "k_replicated" if st.get("replicated_launches", 0) >= max(
         1, st["persistent_launches"] - st.get("replicated_launches", 0)) else "k_persistent"
+    persist_flops, ml_flops, p2_flops = kernel_flops(split, args.steps, pk_name)
     kernels = {
         pk_name: (persist_flops, st["ms_persistent"]),
         "k_eval": (ml_flops, st["ms_eval"]),
@@ -770,7 +794,7 @@ def main() -> int:
     }
     dom = max(kernels, key=lambda k: kernels[k][1])
     dom_flops, dom_ms = kernels[dom]
-    achieved = dom_flops / (dom_ms / 1e3) / 1e12 if dom_ms > 0 else None
+    achieved = dom_flops / (dom_ms / 1e3) / 1e12 if dom_ms > 0 and dom_flops is not None else None
     peak = cub.fp64_peak(local) if rank == 0 else None
     peak_dgemm = measure_fp64_peak(torch) if rank == 0 else None
 
@@ -826,8 +850,9 @@ def main() -> int:
                          "peak_dgemm": peak_dgemm,
                          "peak_dgemm_source": "in-run cuBLAS DGEMM 8192^3 (FP64 tensor path)",
                          "kernel_ms_per_step": {k: v[1] / args.steps for k, v in kernels.items()},
-                         "algorithmic_flops_per_step": {k: v[0] / args.steps
-                                                        for k, v in kernels.items()},
+                         "algorithmic_flops_per_step": {
+                             k: None if v[0] is None else v[0] / args.steps
+                             for k, v in kernels.items()},
                          "regions_per_step": {pk_name: sum(v[0] for v in split.values()),
                                               "k_eval": sum(v[1] for v in split.values()),
                                               "k_phase2": sum(v[2] for v in split.values())},
