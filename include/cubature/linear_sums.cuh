@@ -26,10 +26,13 @@ constexpr double kRound3 = 3.4e-16;  // three units of rounding (2^-53), rounded
 
 // b += a x, with what the rounding of the product and the sum leaves out
 // added to lo: an error of the centre's argument is shared by all points of
-// the region and does not average out as the points' own do.
+// the region and does not average out as the points' own do.  (Intrinsics: a
+// contraction of the residual's terms would count the product's rounding
+// twice.)
 __device__ __forceinline__ void add_product(double& b, double& lo, double a, double x) {
-  const double p = a * x, s = b + p, v = s - b;
-  lo += fma(a, x, -p) + ((b - (s - v)) + (p - v));
+  const double p = __dmul_rn(a, x), s = __dadd_rn(b, p), v = __dadd_rn(s, -b);
+  const double rest = __dadd_rn(__dadd_rn(b, -__dadd_rn(s, -v)), __dadd_rn(p, -v));
+  lo = __dadd_rn(lo, __dadd_rn(fma(a, x, -p), rest));
   b = s;
 }
 
@@ -54,6 +57,12 @@ template <int N>
 struct ThreadSums<CornerPeak<N>> {
   static constexpr bool value = true;
   static constexpr int kMinList = 2048 * (N - 2);
+  // An argument beyond the range of a double becomes the largest one: a point's
+  // value is 0 either way, and the difference of two infinities is no number.
+  __device__ __forceinline__ static double finite(double x) {
+    constexpr double kMax = 1.7976931348623157e308;
+    return fabs(x) > kMax ? copysign(kMax, x) : x;
+  }
   // (b + s)^-(N+1) + (b - s)^-(N+1); two divisions where the product of the
   // powers leaves the normal range
   __device__ __forceinline__ static double pair(double b, double s) {
@@ -68,8 +77,12 @@ struct ThreadSums<CornerPeak<N>> {
     for (int i = 0; i < N; ++i) {
       add_product(b, lo, f.a[i], fma(0.5, H[i], L[i]));
       mag += fabs(f.a[i]) * fmax(fabs(L[i]), fabs(L[i] + H[i]));
-      t[i] = f.a[i] * H[i];
+      t[i] = finite(f.a[i] * H[i]);
       top = fmax(top, fabs(t[i]));
+    }
+    if (finite(b) != b) {
+      b = finite(b);
+      lo = 0;
     }
     const double f0 = 1 / int_power<N + 1>(b);
     double S1 = 0, S2 = 0, S3 = 0, S4 = 0, S5 = 0, S6 = 0, S7 = 0, S8 = 0;
@@ -113,7 +126,10 @@ struct ThreadSums<CornerPeak<N>> {
         S8 += (pair(b, p + l) + pair(b, p - l)) + (pair(b, q + l) + pair(b, q - l));
       }
     }
-    // the argument's centre is b + lo: a relative change of -(N + 1) lo / b
+    // The argument's centre is b + lo: a relative change of -(N + 1) lo / b for
+    // the centre, of -(N + 1) lo / (b + s) for a point.  Taken for all of them:
+    // a point with a smaller argument keeps part of its error, one with a larger
+    // argument is left with at most the centre's on a value below the centre's.
     const double corr = fma(-(N + 1.0) * lo, 1 / b, 1.0);
     out.S[0] = f0 * corr;
     out.S[1] = S1 * corr;

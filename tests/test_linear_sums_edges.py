@@ -1,5 +1,5 @@
-"""Coefficients that the thread-per-region form of continuous has to treat
-apart, against the point-by-point oracle."""
+"""Coefficients that the thread-per-region forms of continuous and corner peak
+have to treat apart, against the point-by-point oracle."""
 import numpy as np
 import pytest
 
@@ -71,3 +71,21 @@ def test_growing_axes_cost_what_the_others_do(cub, ctx):
 
     best(2.0)
     assert best(-2.0) <= 2 * best(2.0)
+
+
+@pytest.mark.parametrize("n,m", [(2, 100), (4, 4200), (8, 12400)])
+def test_corner_peak_arguments_beyond_the_range(cub, oracle, ctx, n, m):
+    """a x is infinite in all or some of the boxes: the values there are zero."""
+    a = [1e308] + [1.0] * (n - 1)
+    lo, ln = _boxes(n, m, n)
+    lo[0] += np.where(np.arange(m) % 2, 5.0, 0.0)
+    ln[0] *= np.where(np.arange(m) % 3, 8.0, 1.0)
+    o = oracle.Rule(n).phase1_eval(oracle.make_integrand("corner_peak", n, a, [0.0] * n), lo, ln,
+                                   1e-4, 1e-12)
+    avg, err, axis, active = [t.cpu().numpy()
+                              for t in _eval(cub, "corner_peak", n, a, [0.0] * n, lo, ln)]
+    assert np.isfinite(o["avg"]).all() and (o["avg"] == 0).any()
+    scale = np.abs(o["avg"]) + o["mag"]
+    assert np.all(np.abs(avg - o["avg"]) <= 1e-13 * scale + 1e-300)
+    assert np.all(np.abs(err - o["err"]) <= 1e-12 * scale + 1e-12 * o["err"] + 1e-300)
+    assert np.array_equal(active, o["active"])
