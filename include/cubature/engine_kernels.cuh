@@ -636,15 +636,19 @@ __device__ __forceinline__ void split_chunk_warp(const EngineArgs& a, long long 
 }
 
 // Padding ids of integral k's next segment, and the segment hand-over
-// (the next list becomes current).
+// (the next list becomes current).  A stopped integral's empty segment keeps
+// its place among the others: the replicated kernel, which may take the list
+// over from here, finds a slot's owner as the last integral that starts at or
+// before it (rep_slot_owner).  With the segment left where it was, such an
+// integral owned slots of the running ones.
 __device__ __forceinline__ void finish_integral(const EngineArgs& a, int k) {
   IntegralState& is = a.ist[k];
   if (is.next_count > 0) {
     const int padded = (is.next_count + 31) & ~31;
     for (int j = is.next_count; j < padded; ++j) a.nrid[is.next_start + j] = -1;
   }
+  is.seg_start = is.next_start;
   if (is.state == kStateRunning) {
-    is.seg_start = is.next_start;
     is.seg_count = is.next_count;
     if (is.next_count == 0) is.state = kStateDone;
   } else {
