@@ -1086,14 +1086,19 @@ struct Phase2Launch {
   bool smem_heap = false;
   size_t heap_smem = 0;
 
-  bool wide = false;
+  SplitForm form = kSplitNarrow;
 
   bool reserve(Workspace& ws, const Options& opt, long long boxes, int sms) {
     int per_sm = 0;
     if constexpr (kSplit) {
-      wide = boxes <= kSplitWideBoxes;
-      return wide ? reserve_split<kSplitLanes<N, true>>(ws, opt, boxes, sms)
-                  : reserve_split<kSplitLanes<N, false>>(ws, opt, boxes, sms);
+      form = boxes <= kSplitFewBoxes    ? kSplitFew
+             : boxes <= kSplitWideBoxes ? kSplitWide
+                                        : kSplitNarrow;
+      switch (form) {
+        case kSplitFew: return reserve_split<kSplitLanes<N, kSplitFew>>(ws, opt, boxes, sms);
+        case kSplitWide: return reserve_split<kSplitLanes<N, kSplitWide>>(ws, opt, boxes, sms);
+        default: return reserve_split<kSplitLanes<N, kSplitNarrow>>(ws, opt, boxes, sms);
+      }
     } else {
       // the heaps in shared memory when two blocks of them fit on an SM (the
       // default 2048 bisections: 98 KB a block), else in the global slab
@@ -1118,10 +1123,11 @@ struct Phase2Launch {
 
   void run(const Src& src, const RuleTables& T, const Phase2Args& p, cudaStream_t s) const {
     if constexpr (kSplit) {
-      if (wide)
-        run_split<kSplitLanes<N, true>>(src, T, p, s);
-      else
-        run_split<kSplitLanes<N, false>>(src, T, p, s);
+      switch (form) {
+        case kSplitFew: return run_split<kSplitLanes<N, kSplitFew>>(src, T, p, s);
+        case kSplitWide: return run_split<kSplitLanes<N, kSplitWide>>(src, T, p, s);
+        default: return run_split<kSplitLanes<N, kSplitNarrow>>(src, T, p, s);
+      }
     } else {
       if (smem_heap)
         k_phase2<N, Src, true><<<(unsigned)blocks, 128, heap_smem, s>>>(src, T, p);

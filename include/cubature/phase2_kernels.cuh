@@ -520,22 +520,37 @@ struct SubBox {
 // are dealt to them).  Few lanes per box give throughput, many a short chain
 // of dependent bisections: up to kSplitWideBoxes boxes (one integral's
 // leftovers, whose longest box sets the end) take the wide form, more the
-// narrow one; up to 4 dimensions there is one form.  Both give a box the same
-// bits (axis_split_sums), so its result does not depend on the choice.
-// Measured on a B200, 8 against 4 lanes: 30 k boxes of a 5-D
-// product peak 1.11 against 1.45 ms, 2.0 M boxes of 6-D ones 62.6 against
-// 55.3 ms.
+// narrow one.  Up to 4 dimensions these two are one, and up to kSplitFewBoxes
+// boxes take 16 lanes per child, a warp per box: the lanes share an axis'
+// factors, and a heap of 1023 entries fits in shared memory.  All forms give a
+// box the same bits (axis_split_sums), so its result does not depend on the
+// choice.
+//
+// Measured on a B200, 8 against 4 lanes: 30 k boxes of a 5-D product peak 1.11
+// against 1.45 ms, 2.0 M boxes of 6-D ones 62.6 against 55.3 ms.  16 against 4
+// (2) lanes in 2 to 4 dimensions, over 250 sets of boxes: 0.63 to 0.94 of the
+// time where the longest boxes set the end, as in most sets of up to 16 k
+// boxes (512 boxes of a 4-D product peak 7.3 against 11.2 ms, 16 k boxes 7.9
+// against 11.5), at most 1.08 where all boxes are short (8.9 k boxes of 4-D
+// Gaussians 0.80 against 0.75 ms); 0.76 to 1.4 for 20 k to 60 k boxes, slower
+// beyond.  (With 4 lanes for all, sets of few boxes took up to 1.55 times what
+// k_phase2 did; with 16 they take 0.7 to 1.1.)
 constexpr int kSplitThreads = 128;
-template <int N, bool kWide>
-constexpr int kSplitLanes = N <= 2 ? 2 : (N <= 4 || !kWide) ? 4 : 8;
+enum SplitForm { kSplitNarrow, kSplitWide, kSplitFew };
+template <int N, SplitForm kForm>
+constexpr int kSplitLanes = N <= 4 && kForm == kSplitFew      ? 16
+                            : N <= 2                          ? 2
+                            : N <= 4 || kForm == kSplitNarrow ? 4
+                                                              : 8;
 constexpr long long kSplitWideBoxes = 1 << 16;
+constexpr long long kSplitFewBoxes = 1 << 14;
 // Heap entries in shared memory and blocks per SM: narrow groups have twice
 // the heaps, and gain from a fifth block (55.5 to 51.6 ms on the 2.0 M boxes;
 // the wide form lost 7% with the smaller heap and fewer registers).
 template <int K>
-constexpr int kSplitTop = K == 8 ? 255 : 127;
+constexpr int kSplitTop = K == 16 ? 1023 : K == 8 ? 255 : 127;
 template <int K>
-constexpr int kSplitBlocks = K == 8 ? 4 : 5;
+constexpr int kSplitBlocks = K >= 8 ? 4 : 5;
 template <int K>
 using SplitHeapOf = detail::SplitHeap<kSplitTop<K>>;
 template <int K>

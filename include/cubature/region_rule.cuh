@@ -316,9 +316,16 @@ struct AxisChoice {
 
   template <int K>
   __device__ __forceinline__ void join_lanes(unsigned mask, int off) {
-    const double ob = __shfl_xor_sync(mask, best, off, K), os = __shfl_xor_sync(mask, second, off, K);
-    const int oa = __shfl_xor_sync(mask, axis, off, K);
-    scale = fmax(scale, __shfl_xor_sync(mask, scale, off, K));
+    join(__shfl_xor_sync(mask, best, off, K), __shfl_xor_sync(mask, second, off, K),
+         __shfl_xor_sync(mask, axis, off, K), __shfl_xor_sync(mask, scale, off, K));
+  }
+  template <int K>
+  __device__ __forceinline__ void join_down(unsigned mask, int off) {
+    join(__shfl_down_sync(mask, best, off, K), __shfl_down_sync(mask, second, off, K),
+         __shfl_down_sync(mask, axis, off, K), __shfl_down_sync(mask, scale, off, K));
+  }
+  __device__ __forceinline__ void join(double ob, double os, int oa, double oscale) {
+    scale = fmax(scale, oscale);
     const double m = second <= os ? os : second, lo = ob <= best ? ob : best;
     second = m <= lo ? lo : m;
     if (ob > best) {
@@ -432,6 +439,18 @@ __device__ __noinline__ int exact_axis_points(const F& f, const double (&L)[N],
 //
 // V: the functor, or a view of its parameters (axis(i)); F: the functor's
 // type.  jac receives the box volume.
+//
+// What one axis adds to the sums, from its factors.
+template <class F>
+__device__ __forceinline__ void append_factors(int d, double tc, double c, double s, double w,
+                                               double p, double q, double l, double len,
+                                               double ratio, AxisPoly& poly, AxisChoice& ch,
+                                               double& vol) {
+  ch.add(d, F::inverse(tc, c), c, s, w, ratio);
+  poly.append(c, s, w, p, q, l);
+  vol = __dmul_rn(vol, len);
+}
+
 template <class F, class V, class Box>
 __device__ __forceinline__ void append_axis(const V& f, const Box& box, int d, double ratio,
                                             AxisPoly& poly, AxisChoice& ch, double& vol) {
@@ -441,11 +460,51 @@ __device__ __forceinline__ void append_axis(const V& f, const Box& box, int d, d
   const double tc = ax.term(fma(0.5, Hd, Ld)), c = F::factor(tc);
   const double s = F::factor2(at(kGenA1, false), at(kGenA1, true));
   const double w = F::factor2(at(kGenA2, false), at(kGenA2, true));
-  ch.add(d, F::inverse(tc, c), c, s, w, ratio);
-  poly.append(c, s, w, F::factor2(at(kGenA3, false), at(kGenA3, true)),
-              F::factor2(at(kGenA4, false), at(kGenA4, true)),
-              F::factor2(at(kGenL, false), at(kGenL, true)));
-  vol = __dmul_rn(vol, Hd);
+  append_factors<F>(d, tc, c, s, w, F::factor2(at(kGenA3, false), at(kGenA3, true)),
+                    F::factor2(at(kGenA4, false), at(kGenA4, true)),
+                    F::factor2(at(kGenL, false), at(kGenL, true)), Hd, ratio, poly, ch, vol);
+}
+
+// Lanes to an axis with K lanes to a region: with 16, what the axes leave room
+// for, up to one for each of the five sums.
+constexpr int split_share(int n, int k) { return k < 16 ? 1 : k / n < 5 ? k / n : 5; }
+
+// append_axis of axis j / R by R lanes (j: lane in the K-lane group): the five
+// sums are dealt to them, and every lane appends all of the axis.
+template <int N, int K, int R, class F, class V, class Box>
+__device__ __forceinline__ void append_axis_lanes(const V& f, const Box& box, int j, unsigned mask,
+                                                  double ratio, AxisPoly& poly, AxisChoice& ch,
+                                                  double& vol) {
+  constexpr int kRounds = (5 + R - 1) / R;
+  const int d = j / R, first = d < N ? d * R : 0;
+  double tc = 0, c = 0, len = 0, v[kRounds];
+#pragma unroll
+  for (int a = 0; a < kRounds; ++a) v[a] = 0;
+  if (d < N) {
+    const auto ax = f.axis(d);
+    const double Ld = box.lo(d);
+    len = box.len(d);
+    tc = ax.term(fma(0.5, len, Ld));
+    c = F::factor(tc);
+#pragma unroll
+    for (int a = 0; a < kRounds; ++a) {
+      const int item = j - first + a * R;
+      const double g = item == 0   ? kGenA1
+                       : item == 1 ? kGenA2
+                       : item == 2 ? kGenA3
+                       : item == 3 ? kGenA4
+                                   : kGenL;
+      if (item < 5)
+        v[a] = F::factor2(ax.term(fma(coef(g, false), len, Ld)),
+                          ax.term(fma(coef(g, true), len, Ld)));
+    }
+  }
+  __syncwarp(mask);
+  double all[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) all[i] = __shfl_sync(mask, v[i / R], first + i % R, K);
+  if (d < N)
+    append_factors<F>(d, tc, c, all[0], all[1], all[2], all[3], all[4], len, ratio, poly, ch, vol);
 }
 
 template <int N, class F, class V, class Box>
@@ -472,7 +531,8 @@ __device__ __forceinline__ void axis_product_sums(const V& f, const Box& box, do
 // leaves out are products with zeros), and lanes of two axes start with the
 // pairs that lanes of one axis join first.  So a box is refined the same way
 // whichever K its call takes.  (With axes j and j + K on lane j the last bits
-// changed with K.)
+// changed with K.)  With several lanes to an axis (K = 16) the lanes of an axis
+// share its factors, and the joins are those of a lane per axis.
 template <int N, int K, class F, class V, class Box>
 __device__ __forceinline__ void axis_split_sums(const V& f, const Box& box, int j, unsigned mask,
                                                 double ratio, RegionSums& out, double& jac) {
@@ -481,21 +541,41 @@ __device__ __forceinline__ void axis_split_sums(const V& f, const Box& box, int 
   jac = 1;
   constexpr int kPer = (N + K - 1) / K;
   static_assert(kPer <= 2, "the joins' order depends on K");
-  const int d1 = (j + 1) * kPer < N ? (j + 1) * kPer : N;
+  constexpr int kShare = split_share(N, K);
+  if constexpr (kShare > 1) {
+    append_axis_lanes<N, K, kShare, F>(f, box, j, mask, ratio, poly, ch, jac);
+#pragma unroll
+    for (int off = kShare; off < N * kShare; off <<= 1) {
+      poly.template join_down<K>(mask, off);
+      ch.template join_down<K>(mask, off);
+      jac = __dmul_rn(jac, __shfl_down_sync(mask, jac, off, K));
+    }
+    // complete in lane 0
+    poly.store(out);
+    out.best = ch.best;
+    out.axis = ch.sure(F::noise(poly.z), poly.z) ? ch.axis : -2;
+#pragma unroll
+    for (int k = 0; k < kNumSets; ++k) out.S[k] = __shfl_sync(mask, out.S[k], 0, K);
+    jac = __shfl_sync(mask, jac, 0, K);
+    out.axis = __shfl_sync(mask, out.axis, 0, K);
+    if (out.axis == -2) out.axis = exact_axis<N, F>(f, box, ratio);
+  } else {
+    const int d1 = (j + 1) * kPer < N ? (j + 1) * kPer : N;
 #pragma unroll 1
-  for (int d = j * kPer; d < d1; ++d) append_axis<F>(f, box, d, ratio, poly, ch, jac);
-  __syncwarp(mask);
+    for (int d = j * kPer; d < d1; ++d) append_axis<F>(f, box, d, ratio, poly, ch, jac);
+    __syncwarp(mask);
 #pragma unroll
-  for (int off = 1; off < K; off <<= 1) {
-    poly.template join_down<K>(mask, off);
-    ch.template join_lanes<K>(mask, off);
-    jac = __dmul_rn(jac, __shfl_xor_sync(mask, jac, off));
+    for (int off = 1; off < K; off <<= 1) {
+      poly.template join_down<K>(mask, off);
+      ch.template join_lanes<K>(mask, off);
+      jac = __dmul_rn(jac, __shfl_xor_sync(mask, jac, off));
+    }
+    poly.store(out);
+#pragma unroll
+    for (int k = 0; k < kNumSets; ++k) out.S[k] = __shfl_sync(mask, out.S[k], 0, K);
+    out.best = ch.best;
+    out.axis = ch.sure(F::noise(out.S[0]), out.S[0]) ? ch.axis : exact_axis<N, F>(f, box, ratio);
   }
-  poly.store(out);
-#pragma unroll
-  for (int k = 0; k < kNumSets; ++k) out.S[k] = __shfl_sync(mask, out.S[k], 0, K);
-  out.best = ch.best;
-  out.axis = ch.sure(F::noise(out.S[0]), out.S[0]) ? ch.axis : exact_axis<N, F>(f, box, ratio);
 }
 
 // A box in an SoA region list.

@@ -1,8 +1,9 @@
 """The second phase of product integrands gives a box the same result however
 many boxes share the call.
 
-Up to 65 536 boxes take 8 lanes per child (n >= 5), more boxes 4: whichever
-form refines a box, its bisections and its bits are the same, so an integral's
+Up to 65 536 boxes take 8 lanes per child (n >= 5), more boxes 4; in 2 to 4
+dimensions up to 16 384 boxes take 16 lanes, more 4 or 2: whichever form refines
+a box, its bisections and its bits are the same, so an integral's
 counts and status do not depend on its batch neighbours or on the number of
 shares of its leftover list.  Values and errors are sums over the boxes, per
 integral in the order of its own boxes: the same bits too.
@@ -41,6 +42,24 @@ def test_integral_alone_and_in_a_batch(cub, ctx, family, n, eps):
         one = ctx.integrate_batch(family, n, [params[k]], eps, 1e-15, opts)[0]
         assert 0 < ctx.stats()["phase2_boxes"] < MANY
         assert one == batch[k], (family, n, k)
+
+
+@pytest.mark.parametrize("family,a", [("product_peak", (15, 25)), ("gaussian", (9, 12))])
+@pytest.mark.parametrize("n,eps,cap,count", [(2, 1e-11, 400, 60), (3, 1e-10, 800, 24),
+                                             (4, 1e-7, 800, 24)])
+def test_integral_alone_and_in_a_batch_low_dimensions(cub, ctx, family, a, n, eps, cap, count):
+    rng = np.random.default_rng(10 * n)
+    params = [cub.make_params(n, list(rng.uniform(*a, n)), list(rng.uniform(0.3, 0.7, n)))
+              for _ in range(count)]
+    opts = cub.options(phase1_cap=cap, persistent=False)
+    ctx.reset_stats()
+    batch = ctx.integrate_batch(family, n, params, eps, 1e-14, opts)
+    assert ctx.stats()["phase2_boxes"] > 1 << 14
+    ctx.reset_stats()
+    for k in (0, 11, count - 1):
+        one = ctx.integrate_batch(family, n, [params[k]], eps, 1e-14, opts)[0]
+        assert one == batch[k], (family, n, k)
+    assert 0 < ctx.stats()["phase2_boxes"] < 1 << 14
 
 
 @pytest.mark.parametrize("cap", [126, 127, 128, 129])
