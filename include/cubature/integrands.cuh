@@ -244,8 +244,10 @@ struct CosSum {
 };
 
 // One integrand of any built-in family, chosen per integral: the family's
-// functor is built once (per region, by the source) and called unchanged,
-// so a mixed batch computes exactly what single-family batches compute.
+// functor is built once (per region, by the source) and called point by point.
+// Single-family batches sum the factored families from factors on long lists
+// and products in the second phase, so a mixed batch agrees with them to
+// rounding there (the points' values are the same).
 template <int N>
 struct MixedGenz {
   int family;
