@@ -11,9 +11,10 @@
 // than the rounding, else from the points (exact_axis_points).
 //
 // Oscillatory would factor too (2 cos b cos t per pair of points, 18 to 37
-// times faster), and more exactly than its points; it stays point by point
-// because the error estimate of a smooth small region is then the rounding of
-// its points, and 1e-9 of the estimates would change.
+// times faster) and more exactly, but is evaluated point by point: where it is
+// smooth over a small region the error estimate is nothing but the rounding of
+// the points, and the exact form would change such estimates by about 1e-9 of
+// the value, and with them which regions are finished at tolerances that low.
 #pragma once
 
 #include "integrands.cuh"

@@ -973,7 +973,11 @@ __device__ __forceinline__ void eval_step(const Src& src, const RuleTables& T, c
 // pass of the groups: a warp per chunk, a thread per slot.  The thread sets up
 // its region as a group does, writes it into the list and evaluates it from
 // there; the chunk's partial is summed on the spot.  A 4-D list of 15 k
-// regions took the groups of 32 lanes seven passes of 10 us.
+// regions took the groups of 32 lanes seven passes of 10 us.  (Corner peak in 7
+// and 8 dimensions needs longer lists than this kernel keeps.)
+template <class F>
+constexpr bool kThreadStep = kFactored<F> && 2 * ThreadSums<F>::kMinList < 32 * kStageChunks;
+
 template <int N, class Src>
 __device__ __forceinline__ void eval_step_threads(const Src& src, const RuleTables& T,
                                                   const EngineArgs& a, const PersistArgs& pa,
@@ -1140,7 +1144,7 @@ __global__ void __launch_bounds__(256, 2) k_persistent(Src src, RuleTables T, Pe
     // smallest R (regions per block) that covers the list in one pass
     const long long per_block = (st.n + gridDim.x - 1) / gridDim.x;
     bool threads = false;
-    if constexpr (detail::kFactored<detail::SourceFn<Src>>) {
+    if constexpr (detail::kThreadStep<detail::SourceFn<Src>>) {
       // longer than a pass of the smallest groups (which beat the stand-alone
       // rule's 32 lanes by a factor of two)
       threads = per_block > p.max_r &&

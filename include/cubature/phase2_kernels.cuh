@@ -526,8 +526,10 @@ struct SubBox {
 // box the same bits (axis_split_sums), so its result does not depend on the
 // choice.
 //
-// Measured on a B200, 8 against 4 lanes: 30 k boxes of a 5-D product peak 1.11
-// against 1.45 ms, 2.0 M boxes of 6-D ones 62.6 against 55.3 ms.  16 against 4
+// Measured on a B200, 8 against 4 lanes, whole calls on product peaks: 0.78
+// (5-D, 1.0 ms) to 1.14 (8-D, 8.2 ms) of the time for 30 k boxes, 0.97 and 1.20
+// for 65 k (5-D, 6-D), 0.91 to 1.30 for 80 k to 94 k, 1.1 to 1.4 from 500 k boxes
+// on.  16 against 4
 // (2) lanes in 2 to 4 dimensions, over 250 sets of boxes: 0.63 to 0.94 of the
 // time where the longest boxes set the end, as in most sets of up to 16 k
 // boxes (512 boxes of a 4-D product peak 7.3 against 11.2 ms, 16 k boxes 7.9

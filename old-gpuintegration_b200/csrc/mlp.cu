@@ -625,22 +625,16 @@ struct CvHook {
   // growable scratch (shared by the hook's copies)
   struct Scratch {
     long long rows = 0;
-    bf16 *X = nullptr, *Ha = nullptr, *Hb = nullptr;
-    double* g = nullptr;
+    double* g = nullptr;  // the network at the rule nodes
     void release() {
-      cudaFree(X);
-      cudaFree(Ha);
-      cudaFree(Hb);
       cudaFree(g);
-      X = Ha = Hb = nullptr;
       g = nullptr;
       rows = 0;
     }
   };
   Scratch* sc;
 
-  // Node rows per chunk: the network's activations for 2^22 rows take
-  // 2 x 1 GB, whatever the length of the list.
+  // Node rows per chunk: 32 MB of values, whatever the length of the list.
   static constexpr long long kRowsMax = 1ll << 22;
 
   int eval(const EngineArgs& a, long long n, cudaStream_t s) const {
