@@ -439,18 +439,6 @@ __device__ __noinline__ int exact_axis_points(const F& f, const double (&L)[N],
 //
 // V: the functor, or a view of its parameters (axis(i)); F: the functor's
 // type.  jac receives the box volume.
-//
-// What one axis adds to the sums, from its factors.
-template <class F>
-__device__ __forceinline__ void append_factors(int d, double tc, double c, double s, double w,
-                                               double p, double q, double l, double len,
-                                               double ratio, AxisPoly& poly, AxisChoice& ch,
-                                               double& vol) {
-  ch.add(d, F::inverse(tc, c), c, s, w, ratio);
-  poly.append(c, s, w, p, q, l);
-  vol = __dmul_rn(vol, len);
-}
-
 template <class F, class V, class Box>
 __device__ __forceinline__ void append_axis(const V& f, const Box& box, int d, double ratio,
                                             AxisPoly& poly, AxisChoice& ch, double& vol) {
@@ -460,9 +448,11 @@ __device__ __forceinline__ void append_axis(const V& f, const Box& box, int d, d
   const double tc = ax.term(fma(0.5, Hd, Ld)), c = F::factor(tc);
   const double s = F::factor2(at(kGenA1, false), at(kGenA1, true));
   const double w = F::factor2(at(kGenA2, false), at(kGenA2, true));
-  append_factors<F>(d, tc, c, s, w, F::factor2(at(kGenA3, false), at(kGenA3, true)),
-                    F::factor2(at(kGenA4, false), at(kGenA4, true)),
-                    F::factor2(at(kGenL, false), at(kGenL, true)), Hd, ratio, poly, ch, vol);
+  ch.add(d, F::inverse(tc, c), c, s, w, ratio);
+  poly.append(c, s, w, F::factor2(at(kGenA3, false), at(kGenA3, true)),
+              F::factor2(at(kGenA4, false), at(kGenA4, true)),
+              F::factor2(at(kGenL, false), at(kGenL, true)));
+  vol = __dmul_rn(vol, Hd);
 }
 
 // Lanes to an axis with K lanes to a region: with 16, what the axes leave room
@@ -503,8 +493,11 @@ __device__ __forceinline__ void append_axis_lanes(const V& f, const Box& box, in
   double all[5];
 #pragma unroll
   for (int i = 0; i < 5; ++i) all[i] = __shfl_sync(mask, v[i / R], first + i % R, K);
-  if (d < N)
-    append_factors<F>(d, tc, c, all[0], all[1], all[2], all[3], all[4], len, ratio, poly, ch, vol);
+  if (d < N) {
+    ch.add(d, F::inverse(tc, c), c, all[0], all[1], ratio);
+    poly.append(c, all[0], all[1], all[2], all[3], all[4]);
+    vol = __dmul_rn(vol, len);
+  }
 }
 
 template <int N, class F, class V, class Box>
